@@ -736,6 +736,8 @@ static bool update_tma_try(const UpdateArgs &a, DevStatus *st, cudaStream_t s, c
 
 // update_tc.cu: the tcgen05 path (FP32 operands split into bf16 planes)
 bool update_tc_try(const UpdateArgs &a, DevStatus *st, cudaStream_t s, cudaError_t &err);
+// f64_update_tc.cu: the FP64 path on the tensor cores (exact digit products)
+bool f64_update_tc_try(const UpdateArgs &a, DevStatus *st, cudaStream_t s, cudaError_t &err);
 
 template <typename T>
 cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st) {
@@ -744,6 +746,11 @@ cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st)
     cudaError_t e = cudaSuccess;
     if (update_tc_try(a, st, s, e)) return e;
     if (update_tma_try(a, st, s, e)) return e;
+  } else if (a.N > 8) {
+    // a tile of the FMA kernel (128 x 64 x 32) takes 66 us of an SM at the FP64
+    // rate, four of the tensor-core kernel's tiles 10: from one column tile on
+    cudaError_t e = cudaSuccess;
+    if (f64_update_tc_try(a, st, s, e)) return e;
   }
   const int nrt = ceil_div(a.M, kUpdBM), nct = ceil_div(a.N, kUpdBN);
   const long long nblk = (long long)nrt * nct * a.nbatch;

@@ -90,6 +90,9 @@ __device__ __forceinline__ void tc_ld4(unsigned taddr, unsigned (&v)[4]) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
                : "r"(taddr));
 }
+__device__ __forceinline__ void tc_ld2(unsigned taddr, unsigned (&v)[2]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(taddr));
+}
 // Each thread of the warp writes 4 consecutive columns of its lane (the
 // warp's quarter of the lanes); tc_wait_st makes the writes complete.
 __device__ __forceinline__ void tc_st4(unsigned taddr, const uint4 &v) {

@@ -1,0 +1,115 @@
+"""FP64 products on the tensor cores (exact digit products, csrc/f64_tc.cuh)
+against quadruple precision, at the edges of their tiles.
+
+Bound: the digit products are exact and the operands rounded below FP64's own
+rounding, so the result may be no further off (relative 2-norm) than the FP64
+FMA path on the same data, or than one correct rounding (2^-53) where that is
+more."""
+import os
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+HALF_ULP = 2.0 ** -53
+
+
+@pytest.fixture()
+def lib():
+    import fastsolver2_gb300 as fs
+    return fs
+
+
+def col(a):
+    return torch.from_numpy(np.ascontiguousarray(np.asarray(a).T)).cuda().t()
+
+
+def both_paths(f):
+    """f() with the tensor cores and with the FP64 FMA kernels."""
+    old = os.environ.get("HODLR_NO_TCGEN05")
+    out = []
+    try:
+        for off in ("0", "1"):
+            os.environ["HODLR_NO_TCGEN05"] = off
+            out.append(f())
+    finally:
+        if old is None:
+            del os.environ["HODLR_NO_TCGEN05"]
+        else:
+            os.environ["HODLR_NO_TCGEN05"] = old
+    return out
+
+
+def rel_err(x, exact):
+    d = (x.astype(np.longdouble) - exact).astype(np.float64)
+    return np.linalg.norm(d) / np.linalg.norm(exact.astype(np.float64))
+
+
+def broadcast(fs, npart, nblock, alpha, U, B, W):
+    """hodlr_gemm_broadcast: W + alpha U B."""
+    u, b, w = col(U), col(B), col(W)
+    n, K = U.shape
+    fs.check(fs.lib().hodlr_gemm_broadcast(n, npart, nblock, K, W.shape[1], alpha, u.data_ptr(), n, b.data_ptr(),
+                                           B.shape[0], 1.0, w.data_ptr(), n))
+    return w.cpu().numpy()
+
+
+def exact_broadcast(nblock, alpha, U, B, W):
+    out, per, K = W.astype(np.longdouble), U.shape[0] // nblock, U.shape[1]
+    for i in range(nblock):
+        out[i * per:(i + 1) * per] += np.longdouble(alpha) * (
+            U[i * per:(i + 1) * per].astype(np.longdouble) @ B[i * K:(i + 1) * K].astype(np.longdouble))
+    return out
+
+
+# (rows, partitions, blocks, inner, columns): one tile, tails of 128 rows, 32 columns and
+# 16 / 32 inner values, both inner chunks, blocks that end inside a tile
+@pytest.mark.parametrize("n,npart,nblock,K,N", [(128, 1, 1, 32, 32), (129, 1, 1, 33, 33), (127, 1, 1, 31, 9),
+                                                (300, 3, 3, 17, 64), (640, 5, 1, 1, 65), (4096, 8, 4, 64, 96),
+                                                (64, 1, 1, 48, 63)])
+@pytest.mark.parametrize("kind", ["normal", "uniform"])
+def test_update_no_less_exact_than_fma(lib, n, npart, nblock, K, N, kind):
+    rng = np.random.default_rng(n + K + N)
+    draw = rng.standard_normal if kind == "normal" else rng.random
+    U, B, W = draw((n, K)), draw((nblock * K, N)), draw((n, N))
+    tc, fma = both_paths(lambda: broadcast(lib, npart, nblock, -1.0, U, B, W))
+    exact = exact_broadcast(nblock, -1.0, U, B, W)
+    assert rel_err(tc, exact) <= max(rel_err(fma, exact), HALF_ULP)
+
+
+def test_update_alpha_units_and_zeros(lib):
+    """alpha, an exact factor on the inner index with its inverse on the other
+    operand (other units), zero rows and columns."""
+    rng = np.random.default_rng(5)
+    U, B, W = rng.standard_normal((300, 40)), rng.standard_normal((40, 50)), rng.standard_normal((300, 50))
+    U[7], U[:, 3], B[:, 11] = 0.0, 0.0, 0.0
+    tc, fma = both_paths(lambda: broadcast(lib, 1, 1, 0.375, U, B, W))
+    exact = exact_broadcast(1, 0.375, U, B, W)
+    assert rel_err(tc, exact) <= max(rel_err(fma, exact), HALF_ULP)
+    p = 2.0 ** rng.integers(-60, 60, 40)
+    assert np.array_equal(tc, broadcast(lib, 1, 1, 0.375, U * p, B / p[:, None], W))
+    assert np.array_equal(tc[7], W[7]) and np.array_equal(tc[:, 11], W[:, 11])
+
+
+def test_update_non_finite_stays_in_its_row_and_column(lib):
+    rng = np.random.default_rng(6)
+    U, B, W = rng.standard_normal((200, 20)), rng.standard_normal((20, 40)), rng.standard_normal((200, 40))
+    U[3, 4], B[2, 7] = np.nan, np.inf
+    tc, fma = both_paths(lambda: broadcast(lib, 1, 1, -1.0, U, B, W))
+    ok = np.isfinite(fma)
+    assert np.array_equal(ok, np.isfinite(tc))
+    # entries of size 1 .. 20, sums of 21 terms: 2^-53 x 21 x 20 each way
+    assert np.abs(tc[ok] - fma[ok]).max() <= 2 * 21 * 20 * HALF_ULP
+
+
+def test_update_extreme_scales(lib):
+    """Products far outside the unit range: scaled by exact powers of two."""
+    rng = np.random.default_rng(7)
+    U, B = rng.standard_normal((128, 16)), rng.standard_normal((16, 32))
+    W = np.zeros((128, 32))
+    base = broadcast(lib, 1, 1, 1.0, U, B, W)
+    for ea, eb in ((-500, -400), (500, 400), (-900, 900)):
+        got = broadcast(lib, 1, 1, 1.0, np.ldexp(U, ea), np.ldexp(B, eb), W)
+        assert np.array_equal(got, np.ldexp(base, ea + eb))
