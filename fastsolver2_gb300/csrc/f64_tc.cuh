@@ -174,8 +174,8 @@ __device__ __forceinline__ int dig_cvt(unsigned v) { return __float2int_rn(__uin
 
 // The eight exact diagonal sums of an output as an integer in units of 2^-55
 // of the bound of |a| |b|, rounded at that unit, for groups of at most KM
-// terms (32, 64 or 128): diagonal d is at most KM 2^13 (d + 1) (pairs with a
-// leading digit, at most 64, count half), which tells where dig_int is exact.
+// terms (32, 64 or 128).  Diagonal d is at most KM d 2^14 (a leading digit is
+// at most 64, the others 128), which tells where dig_raw<0> is exact.
 template <int KM, int W>
 __device__ __forceinline__ long long dig_combine(const unsigned (&v)[kDiag][W], int c) {
   // f: the bits of dig_raw, the integer plus kRaw; pairs f_d + 256 f_(d-1) lose their

@@ -21,7 +21,6 @@
 // sides the updates of one factor + solve take 18.8 ms; the FP64 FMA kernel
 // (update_nn_kernel) took 196.
 #include <algorithm>
-#include <cstdlib>
 
 #include "f64_tc.cuh"
 #include "kernels.cuh"
@@ -372,8 +371,6 @@ static cudaError_t launch_kc(const UpdateArgs &a, DevStatus *st, cudaStream_t s)
 }
 
 bool f64_update_tc_try(const UpdateArgs &a, DevStatus *st, cudaStream_t s, cudaError_t &err) {
-  const char *off = getenv("HODLR_NO_TCGEN05");
-  if (off && off[0] == '1') return false;
   if (a.a_trans || a.K < 1 || a.K > 64) return false;
   if ((long long)ceil_div(a.M, 128) * ceil_div(a.N, kDigN) * a.nbatch > (1 << 30)) return false;  // 32-bit tile counts
   err = a.K <= 32 ? launch_kc<1>(a, st, s) : launch_kc<2>(a, st, s);

@@ -17,6 +17,7 @@
 // thread keeps an (RT/8) x 8 register tile; shared-memory rows are padded by
 // one element so the column-wise staging stores are bank-conflict free.
 #include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -426,12 +427,33 @@ static cudaError_t reduce_rt(const T *A, long long lda, const T *X, long long ld
   return cudaGetLastError();
 }
 
+// f64_reduce_tc.cu: FP64 operands on the tensor cores (exact digit products)
+void f64_reduce_tc_plan(long long nrows, int nbatch, int r, int C, int per_sm, int most, int &nchunks,
+                        int &chunk_rows);
+bool f64_reduce_tc_try(const double *V, long long ldv, const double *X, long long ldx, long long nrows, int nbatch,
+                       int r, int C, int chunk_rows, int nchunks, double *dst, const int *skip, DevStatus *st,
+                       cudaStream_t s, cudaError_t &err);
+
+static bool tensor_cores_off() {
+  const char *off = getenv("HODLR_NO_TCGEN05");
+  return off && off[0] == '1';
+}
+
 template <typename T, typename OutT>
 static cudaError_t reduce_dispatch(const T *A, long long lda, const T *X, long long ldx, long long nrows,
                                    int nbatch, int r, int C, OutT *out, double *work, const int *skip,
                                    cudaStream_t s, DevStatus *st) {
   int nchunks, chunk_rows;
   reduce_plan(nrows, nbatch, C, current_tuning().red_ctas_per_sm * kNumSMs, nchunks, chunk_rows);
+  // FP64 on the tensor cores from 9 columns on, the widest the thin FMA tile
+  // takes (up to 8): a 64-column FMA tile of 64 rows and 32 ranks takes 32 us of
+  // an SM, a group of the tensor-core kernel (128 columns) 4
+  const bool f64_tc = sizeof(T) == 8 && C > 8 && !tensor_cores_off();
+  if (f64_tc) {
+    int most, unused;  // the workspace's chunks
+    reduce_plan(nrows, nbatch, C, kMaxRedCtasPerSm * kNumSMs, most, unused);
+    f64_reduce_tc_plan(nrows, nbatch, r, C, current_tuning().red_ctas_per_sm, most, nchunks, chunk_rows);
+  }
   const int bn = red_bn(C);
   const int nct = ceil_div(C, bn);
   cudaError_t e = cudaSuccess;
@@ -444,6 +466,9 @@ static cudaError_t reduce_dispatch(const T *A, long long lda, const T *X, long l
       done = reduce_tc_try<D>(A, lda, X, ldx, nrows, nbatch, r, C, chunk_rows, nchunks, dst, skip, st, s, err);
       if (!done)
         done = reduce_tma_try<D>(A, lda, X, ldx, nrows, nbatch, r, C, chunk_rows, nchunks, dst, skip, st, s, err);
+    } else if constexpr (std::is_same<D, double>::value) {
+      if (f64_tc)
+        done = f64_reduce_tc_try(A, lda, X, ldx, nrows, nbatch, r, C, chunk_rows, nchunks, dst, skip, st, s, err);
     }
     if (done) return err;
 #define HODLR_RED(RTV, BNV) \
@@ -746,7 +771,7 @@ cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st)
     cudaError_t e = cudaSuccess;
     if (update_tc_try(a, st, s, e)) return e;
     if (update_tma_try(a, st, s, e)) return e;
-  } else if (a.N > 8) {
+  } else if (a.N > 8 && !tensor_cores_off()) {
     // a tile of the FMA kernel (128 x 64 x 32) takes 66 us of an SM at the FP64
     // rate, four of the tensor-core kernel's tiles 10: from one column tile on
     cudaError_t e = cudaSuccess;

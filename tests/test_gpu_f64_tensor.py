@@ -113,3 +113,50 @@ def test_update_extreme_scales(lib):
     for ea, eb in ((-500, -400), (500, 400), (-900, 900)):
         got = broadcast(lib, 1, 1, 1.0, np.ldexp(U, ea), np.ldexp(B, eb), W)
         assert np.array_equal(got, np.ldexp(base, ea + eb))
+
+
+def reduce(fs, npart, V, X):
+    """hodlr_gemm_reduce: the partitions' V^T X stacked."""
+    v, x = col(V), col(X)
+    n, r = V.shape
+    w = torch.zeros((X.shape[1], npart * r), dtype=torch.float64, device="cuda").t()
+    fs.check(fs.lib().hodlr_gemm_reduce(n, npart, r, X.shape[1], v.data_ptr(), n, x.data_ptr(), n, w.data_ptr(),
+                                        npart * r))
+    return w.cpu().numpy()
+
+
+def exact_reduce(npart, V, X):
+    per, q = V.shape[0] // npart, np.longdouble
+    return np.concatenate([V[i * per:(i + 1) * per].astype(q).T @ X[i * per:(i + 1) * per].astype(q)
+                           for i in range(npart)])
+
+
+# (rows, partitions, rank, columns): groups of 64 rows and their halves, 32 ranks, 128 columns, row chunks
+@pytest.mark.parametrize("n,npart,r,C", [(64, 1, 32, 128), (65, 1, 33, 129), (63, 1, 31, 9), (96, 3, 1, 65),
+                                         (2000, 2, 16, 40), (5120, 1, 64, 200), (40, 1, 8, 17)])
+@pytest.mark.parametrize("kind", ["normal", "uniform"])
+def test_reduce_no_less_exact_than_fma(lib, n, npart, r, C, kind):
+    rng = np.random.default_rng(n + r + C)
+    draw = rng.standard_normal if kind == "normal" else rng.random
+    V, X = draw((n, r)), draw((n, C))
+    tc, fma = both_paths(lambda: reduce(lib, npart, V, X))
+    exact = exact_reduce(npart, V, X)
+    assert rel_err(tc, exact) <= max(rel_err(fma, exact), HALF_ULP)
+
+
+def test_reduce_units_zeros_and_non_finite(lib):
+    rng = np.random.default_rng(8)
+    V, X = rng.standard_normal((300, 20)), rng.standard_normal((300, 40))
+    V[5], X[9], V[:, 3], X[:, 7] = 0.0, 0.0, 0.0, 0.0
+    tc = reduce(lib, 1, V, X)
+    assert not tc[3].any() and not tc[:, 7].any()
+    p = 2.0 ** rng.integers(-60, 60, 300)
+    assert np.array_equal(tc, reduce(lib, 1, V * p[:, None], X / p[:, None]))
+    V[70, 4], X[200, 11] = np.inf, np.nan
+    bad, fma = both_paths(lambda: reduce(lib, 1, V, X))
+    ok = np.ones_like(bad, dtype=bool)
+    ok[4], ok[:, 11] = False, False
+    assert np.isfinite(bad[ok]).all() and not np.isfinite(bad[~ok]).any()
+    V[70, 4], X[200, 11] = 0.0, 0.0  # in rank 4 and column 11 only: out of the compared entries
+    exact = exact_reduce(1, V, X)
+    assert rel_err(bad[ok], exact[ok]) <= max(rel_err(fma[ok], exact[ok]), HALF_ULP)
