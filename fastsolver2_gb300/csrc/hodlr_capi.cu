@@ -138,6 +138,10 @@ struct hodlr_ctx {
   float *Sinv32 = nullptr;    // mixed mode: FP32 inverses (from the FP64-factored systems)
   double *Dinv = nullptr;     // [nleaf][m][m] leaf inverses (FP64 mode)
   float *Dinv32 = nullptr;    // (mixed mode)
+  // FP64 mode: digit images of the leaf inverses for the tensor-core
+  // application, their row scales and balances (null: FMA kernels only)
+  unsigned char *Dimg = nullptr;
+  int *Drow = nullptr, *Dbal = nullptr;
   bool factored = false;
   // workspaces
   double *Tbuf = nullptr, *Wbuf = nullptr, *eta = nullptr, *red = nullptr;
@@ -480,11 +484,19 @@ template <> double *Dinvptr<double>(hodlr_ctx *h) { return h->Dinv; }
 template <> float *Dinvptr<float>(hodlr_ctx *h) { return h->Dinv32; }
 
 // X := D^{-1} X (or D^{-T} X) on every leaf's rows: explicit inverse GEMM when
-// the leaf size has a tuned kernel, LU triangular solves otherwise.
+// the leaf size has a tuned kernel, LU triangular solves otherwise.  In FP64
+// the forward application takes the tensor cores from kThinCols + 1 columns on:
+// a leaf of 128 and up to 64 columns take 9 us of an SM there (the products),
+// 260 us at the FP64 FMA rate.
+constexpr int kThinCols = 8;
 template <typename T>
 static int leaf_solve(hodlr_ctx *h, T *X, long long ldx, int ncols, bool trans, const int *skip) {
   T *Dinv = Dinvptr<T>(h);
-  if (Dinv)
+  if (sizeof(T) == 8 && h->Dimg && !trans && ncols > kThinCols)
+    PHASE(h, HODLR_PHASE_LEAF_SOLVE,
+          launch_f64_leaf_tc(h->Dimg, h->Drow, h->Dbal, h->m, h->nleaf, reinterpret_cast<const double *>(X), ldx,
+                             reinterpret_cast<double *>(X), ldx, ncols, skip, h->dst, h->st));
+  else if (Dinv)
     PHASE(h, HODLR_PHASE_LEAF_SOLVE,
           launch_leaf_apply<T>(Dinv, h->m, h->nleaf, X, ldx, ncols, trans, skip, h->st));
   else
@@ -593,8 +605,15 @@ template <typename T> static int factor_sweep(hodlr_ctx *h, bool leaves_done = f
       if (Dinv && !fused) PHASE(h, HODLR_PHASE_LEAF_LU, launch_leaf_inverse<T>(LU, h->ipiv, m, h->nleaf, Dinv, s));
     }
   }
+  if (sizeof(T) == 8 && h->Dimg)  // also for the solves
+    PHASE(h, HODLR_PHASE_LEAF_LU,
+          launch_f64_leaf_image(reinterpret_cast<const double *>(Dinv), m, h->nleaf, h->Dimg, h->Drow, h->Dbal, s));
   if (L == 0) return HODLR_OK;
-  if (sizeof(T) == 4 && Dinv && m == 128) {
+  if (sizeof(T) == 8 && h->Dimg) {  // Utilde = D^{-1} U on the tensor cores, straight from U
+    PHASE(h, HODLR_PHASE_LEAF_SOLVE,
+          launch_f64_leaf_tc(h->Dimg, h->Drow, h->Dbal, m, h->nleaf, h->U, n, reinterpret_cast<double *>(Ut), n, L * r,
+                             nullptr, h->dst, s));
+  } else if (sizeof(T) == 4 && Dinv && m == 128) {
     // Utilde = D^{-1} U straight from the FP64 U (rounded as it is split or
     // staged): on the tensor cores, or the FMA tiles when the tuning asks
     PHASE(h, HODLR_PHASE_LEAF_SOLVE,
@@ -1327,6 +1346,21 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
   ALLOC(h->dst, DevStatus, 1);
   ALLOC(h->dst_leaf, DevStatus, 1);
 #undef ALLOC
+  // the digit images last, and only out of plenty: without them the leaf
+  // application runs on the FP64 FMA kernels
+  const char *no_tc64 = getenv("HODLR_NO_TCGEN05");
+  if (h->Dinv && !(no_tc64 && no_tc64[0] == '1')) {
+    const size_t bytes = f64_leaf_image_bytes(m, h->nleaf);
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) == cudaSuccess && bytes <= avail / 4) {
+      cudaError_t ie = cudaSuccess;
+      unsigned char *img = h->alloc<unsigned char>(bytes, ie);
+      if (ie == cudaSuccess) h->Drow = h->alloc<int>(f64_leaf_image_rows(m, h->nleaf), ie);
+      if (ie == cudaSuccess) h->Dbal = h->alloc<int>((size_t)n, ie);
+      if (ie == cudaSuccess) h->Dimg = img;
+    }
+    (void)cudaGetLastError();
+  }
   if (cudaMallocHost(&h->hst, sizeof(DevStatus)) != cudaSuccess) {
     free_ctx(h);
     return set_err(HODLR_ERR_OUT_OF_MEMORY, "cudaMallocHost");
@@ -3054,6 +3088,9 @@ int hodlr_checkpoint_load(const void *buf, int64_t bytes, void *stream, hodlr_ha
   h->leaves_prefactored = false;
   std::fill(h->has_level.begin(), h->has_level.end(), (char)1);
   int rc = prepare_leaves(h);
+  if (rc == HODLR_OK && h->Dimg &&
+      launch_f64_leaf_image(h->Dinv, h->m, h->nleaf, h->Dimg, h->Drow, h->Dbal, h->st) != cudaSuccess)
+    rc = set_err(HODLR_ERR_CUDA, "checkpoint preparation");
   for (int l = 0; l < h->L && rc == HODLR_OK; ++l) rc = prepare_level(h, l);
   if (rc != HODLR_OK) {
     hodlr_destroy(h);

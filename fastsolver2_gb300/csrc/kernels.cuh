@@ -140,6 +140,18 @@ cudaError_t launch_leaf_apply_f64src(const float *Dinv, int m, int nleaf, const 
 bool leaf_apply_tc_try(const float *Dinv, int nleaf, const double *U, long long lds, float *Y, long long ldy,
                        int ncols, DevStatus *st, cudaStream_t s, cudaError_t &err);
 
+// The FP64 application on the tensor cores (f64_leaf_tc.cu, leaf sizes 64, 128
+// and 256): the inverses' digit images, their sizes (plane bytes, ints of row
+// scales; the balances take nleaf * m ints), and Y_i = Dinv_i X_i from them
+// (Y may be X).
+size_t f64_leaf_image_bytes(int m, int nleaf);
+size_t f64_leaf_image_rows(int m, int nleaf);
+cudaError_t launch_f64_leaf_image(const double *Dinv, int m, int nleaf, unsigned char *img, int *rows, int *bal,
+                                  cudaStream_t s);
+cudaError_t launch_f64_leaf_tc(const unsigned char *img, const int *rows, const int *bal, int m, int nleaf,
+                               const double *X, long long ldx, double *Y, long long ldy, int ncols, const int *skip,
+                               DevStatus *st, cudaStream_t s);
+
 // Capacitance factorisation of the nodes of one depth: S from the T blocks'
 // columns [ucol, ucol + r), FP64 LU (stored in cap_lu / cap_ipiv) and the FP64
 // inverse Sinv (plus its double-word split in sinv2 when given).

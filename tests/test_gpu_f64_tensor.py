@@ -160,3 +160,36 @@ def test_reduce_units_zeros_and_non_finite(lib):
     V[70, 4], X[200, 11] = 0.0, 0.0  # in rank 4 and column 11 only: out of the compared entries
     exact = exact_reduce(1, V, X)
     assert rel_err(bad[ok], exact[ok]) <= max(rel_err(fma[ok], exact[ok]), HALF_ULP)
+
+
+# column counts around the 32-column tiles and the pairs of them; two leaves at least
+@pytest.mark.parametrize("m", [64, 128, 256])
+@pytest.mark.parametrize("k", [9, 32, 65])
+def test_leaf_application_no_less_exact_than_fma(lib, m, k):
+    """Leaf solves alone (zero coupling): X = blockdiag(D)^-1 B, in place."""
+    rng = np.random.default_rng(m + k)
+    nl = 4
+    D = rng.standard_normal((nl, m, m)) / np.sqrt(m) + 4.0 * np.eye(m)
+    B = rng.standard_normal((nl * m, k))
+    zero = torch.zeros((1, nl * m), dtype=torch.float64, device="cuda").t()
+
+    def solve():
+        s = lib.Solver(nl * m, m, 2, 1, nrhs_max=k)
+        d = torch.from_numpy(np.ascontiguousarray(D.transpose(0, 2, 1))).cuda()
+        s.set_leaf_blocks(d.reshape(-1), ld=m, leaf_stride=m * m)
+        for l in range(2):
+            s.set_lowrank(l, zero, zero)
+        s.factor()
+        b = col(B)
+        s.solve(b)
+        out = b.cpu().numpy()
+        s.close()
+        return out
+
+    tc, fma = both_paths(solve)
+    q = np.longdouble
+    x = np.concatenate([np.linalg.solve(D[i], B[i * m:(i + 1) * m]) for i in range(nl)]).astype(q)
+    for _ in range(2):  # refined in quadruple precision
+        r = [B[i * m:(i + 1) * m].astype(q) - D[i].astype(q) @ x[i * m:(i + 1) * m] for i in range(nl)]
+        x = x + np.concatenate([np.linalg.solve(D[i], r[i].astype(np.float64)) for i in range(nl)])
+    assert rel_err(tc, x) <= max(rel_err(fma, x), HALF_ULP)
