@@ -271,6 +271,9 @@ template <typename T>
 cudaError_t launch_leaf_apply(const T *Dinv, int m, int nleaf, T *X, long long ldx, int ncols, bool trans,
                               const int *skip, cudaStream_t s) {
   if (ncols <= 0 || nleaf <= 0) return cudaSuccess;
+  if constexpr (std::is_same<T, double>::value) {
+    if (ncols <= 8) return launch_f64_thin_leaf(Dinv, m, nleaf, X, ldx, ncols, trans, skip, s);
+  }
   switch (m) {
     case 64: return leaf_apply_m<T, 64>(Dinv, nleaf, X, ldx, ncols, trans, skip, s);
     case 128: return leaf_apply_m<T, 128>(Dinv, nleaf, X, ldx, ncols, trans, skip, s);
@@ -904,6 +907,7 @@ cudaError_t launch_cap_apply(const CapApplyArgs &a, cudaStream_t s) {
   const int MT = n2 <= 32 ? 1 : (n2 <= 64 ? 2 : 4);
   const int NP = MT * 32;
   const bool dw = a.sinv2 != nullptr;
+  if (!dw && a.C <= 8) return launch_f64_thin_cap(a, s);
   const size_t es = dw ? sizeof(float2) : sizeof(double);
   const size_t bytes = (size_t)NP * NP * es + (size_t)NP * 32 * es;
   // enough CTAs to fill the GPU, each covering several column tiles of its node

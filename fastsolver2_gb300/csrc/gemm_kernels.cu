@@ -474,9 +474,15 @@ static cudaError_t reduce_dispatch(const T *A, long long lda, const T *X, long l
 #define HODLR_RED(RTV, BNV) \
   err = reduce_rt<T, RTV, BNV, D>(A, lda, X, ldx, nrows, nbatch, r, C, chunk_rows, nchunks, nct, dst, skip, s)
     if (bn == 8) {
-      if (r <= 16) HODLR_RED(16, 8);
-      else if (r <= 32) HODLR_RED(32, 8);
-      else HODLR_RED(64, 8);
+      if constexpr (sizeof(T) == 4) {
+        if (r <= 16) HODLR_RED(16, 8);
+        else if (r <= 32) HODLR_RED(32, 8);
+        else HODLR_RED(64, 8);
+      } else if constexpr (std::is_same<D, double>::value) {
+        err = launch_f64_thin_reduce(A, lda, X, ldx, nrows, nbatch, r, C, chunk_rows, nchunks, dst, skip, s);
+      } else {
+        err = cudaErrorInvalidValue;  // FP64 operands give FP64 results
+      }
     } else {
       if (r <= 16) HODLR_RED(16, 64);
       else if (r <= 32) HODLR_RED(32, 64);
@@ -771,11 +777,16 @@ cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st)
     cudaError_t e = cudaSuccess;
     if (update_tc_try(a, st, s, e)) return e;
     if (update_tma_try(a, st, s, e)) return e;
-  } else if (a.N > 8 && !tensor_cores_off()) {
-    // a tile of the FMA kernel (128 x 64 x 32) takes 66 us of an SM at the FP64
-    // rate, four of the tensor-core kernel's tiles 10: from one column tile on
+  } else {
     cudaError_t e = cudaSuccess;
-    if (f64_update_tc_try(a, st, s, e)) return e;
+    if (a.overwrite && (a.K > 4 || a.a_trans)) return cudaErrorInvalidValue;  // the others add to C
+    // Up to 4 columns, or 4 inner values, the FP64 FMAs are few and every value
+    // is read once by the thin kernels; from 5 on a 128 x 32 tile takes 6 us of an
+    // SM on the tensor cores, and 8 columns 8 us on the FMA pipe (rank 32)
+    if (!a.a_trans && a.K <= 4) return launch_f64_thin_outer(a, s);
+    if (!a.a_trans && a.N <= 4) return launch_f64_thin_update(a, s);
+    if (!tensor_cores_off() && f64_update_tc_try(a, st, s, e)) return e;
+    if (!a.a_trans && a.N <= 8) return launch_f64_thin_update(a, s);
   }
   const int nrt = ceil_div(a.M, kUpdBM), nct = ceil_div(a.N, kUpdBN);
   const long long nblk = (long long)nrt * nct * a.nbatch;

@@ -486,9 +486,9 @@ template <> float *Dinvptr<float>(hodlr_ctx *h) { return h->Dinv32; }
 // X := D^{-1} X (or D^{-T} X) on every leaf's rows: explicit inverse GEMM when
 // the leaf size has a tuned kernel, LU triangular solves otherwise.  In FP64
 // the forward application takes the tensor cores from kThinCols + 1 columns on:
-// a leaf of 128 and up to 64 columns take 9 us of an SM there (the products),
-// 260 us at the FP64 FMA rate.
-constexpr int kThinCols = 8;
+// a leaf of 128 and up to 32 columns take 5 us of an SM there, two columns 8 us
+// at the FP64 FMA rate, one 4.
+constexpr int kThinCols = 2;
 template <typename T>
 static int leaf_solve(hodlr_ctx *h, T *X, long long ldx, int ncols, bool trans, const int *skip) {
   T *Dinv = Dinvptr<T>(h);
@@ -1654,9 +1654,11 @@ int hodlr_adjoint(hodlr_handle h, const double *x, int64_t ldx, const double *g,
     return rc;
   }
   cudaStream_t s = h->st;
+  const int ow = k <= 4;  // the products of few columns are written, not added to zeros
   if (gr->dD) {
-    CK(cudaMemsetAsync(gr->dD, 0, sizeof(double) * h->nleaf * m * m, s));
+    if (!ow) CK(cudaMemsetAsync(gr->dD, 0, sizeof(double) * h->nleaf * m * m, s));
     UpdateArgs ua{};
+    ua.overwrite = ow;
     ua.A = lam;
     ua.lda = ldl;
     ua.a_bstride = m;
@@ -1684,8 +1686,9 @@ int hodlr_adjoint(hodlr_handle h, const double *x, int64_t ldx, const double *g,
       double *dst = which == 0 ? gr->dU : gr->dV;
       if (!dst) continue;
       dst += (long long)l * n * r;
-      CK(cudaMemsetAsync(dst, 0, sizeof(double) * n * r, s));
+      if (!ow) CK(cudaMemsetAsync(dst, 0, sizeof(double) * n * r, s));
       UpdateArgs ua{};
+      ua.overwrite = ow;
       ua.A = which == 0 ? lam : x;
       ua.lda = which == 0 ? ldl : ldx;
       ua.a_bstride = rows;

@@ -118,7 +118,17 @@ struct UpdateArgs {
   int M, N, K, nbatch;
   double alpha;
   const int *skip;
+  int overwrite;  // FP64, K <= 4: C_b = instead of += (its old values are not read)
 };
+// f64_thin.cu: the FP64 steps for up to 8 columns (update, reduction, leaf and
+// capacitance application), and updates of an inner dimension up to 4
+cudaError_t launch_f64_thin_update(const UpdateArgs &a, cudaStream_t s);
+cudaError_t launch_f64_thin_outer(const UpdateArgs &a, cudaStream_t s);
+cudaError_t launch_f64_thin_reduce(const double *A, long long lda, const double *X, long long ldx, long long nrows,
+                                   int nbatch, int r, int C, int chunk_rows, int nchunks, double *dst, const int *skip,
+                                   cudaStream_t s);
+cudaError_t launch_f64_thin_leaf(const double *Dinv, int m, int nleaf, double *X, long long ldx, int C, bool trans,
+                                 const int *skip, cudaStream_t s);
 template <typename T>
 cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st = nullptr);
 
@@ -185,6 +195,7 @@ struct CapApplyArgs {
   const int *skip;
 };
 cudaError_t launch_cap_apply(const CapApplyArgs &a, cudaStream_t s);
+cudaError_t launch_f64_thin_cap(const CapApplyArgs &a, cudaStream_t s);  // FP64, up to 8 columns
 
 // --------------------------------------------------------------- helpers
 // Y[i, j] = (T) X[i, j] for an n x c column-major tile.
