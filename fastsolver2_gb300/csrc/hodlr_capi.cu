@@ -191,9 +191,11 @@ struct hodlr_ctx {
   // skips its own leaf LU and takes over that status
   DevStatus *dst_leaf = nullptr;
   bool leaves_prefactored = false;
-  // mixed mode, leaf 128: the factorisation forms only the leaf inverses the
-  // sweeps apply; LU32 / ipiv are formed on request (ensure_leaf_lu)
+  // the factorisation forms only the leaf inverses the sweeps apply (mixed
+  // mode, leaf 128; FP64 mode with digit images); LU32 or LU, and ipiv, are
+  // formed on request (ensure_leaf_lu)
   bool lu_stale = false;
+  bool keep_lu = false;  // FP64: the caller wants the LU factors of every factorisation
   float factor_ms = 0.f, solve_ms = 0.f;
   // graphs
   bool use_graphs = true;
@@ -530,9 +532,13 @@ static int cap_apply(hodlr_ctx *h, int l, int C, long long tb_stride, bool trans
   return HODLR_OK;
 }
 
-// The mixed path at leaf 128 factors its leaves by the blocked Gauss-Jordan
-// kernel, which forms the explicit inverses only.
-static bool leaf_inverse_only(const hodlr_ctx *h) { return h->mixed && h->m == 128 && h->Dinv32; }
+// The mixed path at leaf 128, and the FP64 path where it has digit images,
+// factor their leaves by blocked Gauss-Jordan kernels that form the explicit
+// inverses only.  FP64: 8192 leaves of 128 rows take 15 ms so, and 69 in the
+// register-resident sweep that gives LU and inverse together.
+static bool leaf_inverse_only(const hodlr_ctx *h) {
+  return h->mixed ? h->m == 128 && h->Dinv32 : h->Dimg && !h->keep_lu;
+}
 
 static cudaError_t launch_mixed_leaf_factor(hodlr_ctx *h, DevStatus *st, cudaStream_t s) {
   const int m = h->m;
@@ -545,13 +551,15 @@ static cudaError_t launch_mixed_leaf_factor(hodlr_ctx *h, DevStatus *st, cudaStr
   return e;
 }
 
-// The leaf LU factors and pivots of a factored mixed handle whose
-// factorisation formed only the inverses: formed now, from the leaf blocks.
+// The leaf LU factors and pivots of a factored handle whose factorisation formed only the inverses: formed now, from the leaf blocks.
 static int ensure_leaf_lu(hodlr_ctx *h) {
   if (!h->lu_stale) return HODLR_OK;
   CKS(reset_status(h));
-  CK(launch_leaf_getrf<float>(h->D, h->m, (long long)h->m * h->m, h->LU32, h->ipiv, h->m, h->nleaf, h->dst, nullptr,
-                              h->st));
+  const long long mm = (long long)h->m * h->m;
+  if (h->mixed)
+    CK(launch_leaf_getrf<float>(h->D, h->m, mm, h->LU32, h->ipiv, h->m, h->nleaf, h->dst, nullptr, h->st));
+  else
+    CK(launch_leaf_getrf<double>(h->D, h->m, mm, h->LU, h->ipiv, h->m, h->nleaf, h->dst, nullptr, h->st));
   CKS(sync_status(h, nullptr));
   h->lu_stale = false;
   return HODLR_OK;
@@ -598,6 +606,9 @@ template <typename T> static int factor_sweep(hodlr_ctx *h, bool leaves_done = f
   if (!leaves_done) {
     if (sizeof(T) == 4) {
       PHASE(h, HODLR_PHASE_LEAF_LU, launch_mixed_leaf_factor(h, h->dst, s));
+    } else if (leaf_inverse_only(h)) {  // LU is the workspace, the images' memory the scratch
+      PHASE(h, HODLR_PHASE_LEAF_LU,
+            launch_f64_leaf_gj(h->D, m, (long long)m * m, m, h->nleaf, h->LU, h->ipiv, h->Dinv, h->Dimg, h->dst, s));
     } else {
       PHASE(h, HODLR_PHASE_LEAF_LU,
             launch_leaf_getrf<T>(h->D, m, (long long)m * m, LU, h->ipiv, m, h->nleaf, h->dst, fused ? Dinv : nullptr,
@@ -1350,7 +1361,8 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
   // application runs on the FP64 FMA kernels
   const char *no_tc64 = getenv("HODLR_NO_TCGEN05");
   if (h->Dinv && !(no_tc64 && no_tc64[0] == '1')) {
-    const size_t bytes = f64_leaf_image_bytes(m, h->nleaf);
+    // (the memory is also the scratch of the leaf factorisation)
+    const size_t bytes = std::max(f64_leaf_image_bytes(m, h->nleaf), f64_leaf_gj_scratch(m, h->nleaf));
     size_t avail = 0, total = 0;
     if (cudaMemGetInfo(&avail, &total) == cudaSuccess && bytes <= avail / 4) {
       cudaError_t ie = cudaSuccess;
@@ -1893,6 +1905,8 @@ int hodlr_hsolve_ex(int nrow, int nrhs, int rank, int nPart, int LD, double *K, 
   d.stream = stream;
   hodlr_handle h = nullptr;
   CKS(hodlr_create(&d, &h));
+  // K receives the LU factors: leaves up to 128 rows give LU and inverse in one sweep
+  h->keep_lu = m <= 128;
   double *dK = K, *dU = U, *dV = V;
   long long ld = LD;
   int rc = HODLR_OK;

@@ -193,3 +193,62 @@ def test_leaf_application_no_less_exact_than_fma(lib, m, k):
         r = [B[i * m:(i + 1) * m].astype(q) - D[i].astype(q) @ x[i * m:(i + 1) * m] for i in range(nl)]
         x = x + np.concatenate([np.linalg.solve(D[i], r[i].astype(np.float64)) for i in range(nl)])
     assert rel_err(tc, x) <= max(rel_err(fma, x), HALF_ULP)
+
+
+def factored_leaves(lib, D, B):
+    """X of blockdiag(D) X = B through a solver, and the handle."""
+    nl, m = D.shape[:2]
+    s = lib.Solver(nl * m, m, int(np.log2(nl)), 1, nrhs_max=B.shape[1])
+    d = torch.from_numpy(np.ascontiguousarray(D.transpose(0, 2, 1))).cuda()
+    s.set_leaf_blocks(d.reshape(-1), ld=m, leaf_stride=m * m)
+    zero = torch.zeros((1, nl * m), dtype=torch.float64, device="cuda").t()
+    for l in range(int(np.log2(nl))):
+        s.set_lowrank(l, zero, zero)
+    s.factor()
+    b = col(B)
+    s.solve(b)
+    return b.cpu().numpy(), s
+
+
+@pytest.mark.parametrize("m", [64, 128, 256])
+def test_leaf_inverse_that_pivots(lib, m):
+    """Blocks whose pivots lie far from the diagonal, in every panel: a
+    permutation of rows moves the large entries away.  Bound: an inverse formed
+    by elimination with pivoting and applied, 4 m 2^-53 cond^2."""
+    rng = np.random.default_rng(m)
+    D = np.stack([(rng.standard_normal((m, m)) / np.sqrt(m) + 4.0 * np.eye(m))[rng.permutation(m)] for _ in range(2)])
+    B = rng.standard_normal((2 * m, 3))
+    x, s = factored_leaves(lib, D, B)
+    for i in range(2):
+        exact = np.linalg.solve(D[i], B[i * m:(i + 1) * m])
+        err = np.linalg.norm(x[i * m:(i + 1) * m] - exact) / np.linalg.norm(exact)
+        assert err <= 4 * m * HALF_ULP * np.linalg.cond(D[i]) ** 2
+    # the LU factors and pivots, formed on request: P D = L U
+    lu = torch.zeros(2 * m * m, dtype=torch.float64, device="cuda")
+    piv = torch.zeros(2 * m, dtype=torch.int32, device="cuda")
+    s.get_factors(leaf_lu=lu, leaf_ipiv=piv)
+    lu, piv = lu.cpu().numpy().reshape(2, m, m).transpose(0, 2, 1), piv.cpu().numpy().reshape(2, m)
+    for i in range(2):
+        P = D[i].copy()
+        for k, p in enumerate(piv[i]):
+            P[[k, p - 1]] = P[[p - 1, k]]
+        L, R = np.tril(lu[i], -1) + np.eye(m), np.triu(lu[i])
+        assert (np.abs(P - L @ R) <= 2 * m * HALF_ULP * (np.abs(L) @ np.abs(R))).all()
+
+
+@pytest.mark.parametrize("m", [64, 128, 256])
+@pytest.mark.parametrize("kind", ["equal rows", "zero row", "zero column", "rank one"])
+def test_singular_leaf_is_refused(lib, m, kind):
+    rng = np.random.default_rng(m)
+    D = np.stack([rng.standard_normal((m, m)) for _ in range(2)])
+    if kind == "equal rows":
+        D[1] = np.where(np.arange(m)[:, None] == m - 3, D[1, 2], D[1]) if m != 256 else np.ones((m, m))
+    elif kind == "zero row":
+        D[1, m // 2] = 0.0
+    elif kind == "zero column":
+        D[1, :, m - 1] = 0.0
+    else:
+        D[1] = 1.0
+    with pytest.raises(lib.HodlrError) as e:
+        factored_leaves(lib, D, np.ones((2 * m, 1)))
+    assert e.value.code == lib.HODLR_ERR_SINGULAR_LEAF and "index 1" in str(e.value)
