@@ -10,6 +10,7 @@
 // solves: no per-row synchronisation, full register tiling, and the same
 // flop count as the two triangular solves it replaces.
 #include <algorithm>
+#include <cstdlib>
 #include <type_traits>
 
 #include "dense_ops.cuh"
@@ -290,7 +291,9 @@ template cudaError_t launch_leaf_apply<float>(const float *, int, int, float *, 
 // One CTA per node of a depth: S = [I, s.T1u; s.T0u, I] (FP64), LU with
 // partial pivoting (stored for inspection), then Sinv = S^{-1} (FP64, and a
 // double-word copy when sinv2 is given).
-__global__ void __launch_bounds__(256) cap_factor_kernel(CapFactorArgs a) {
+// `only` (may be null): the nodes of the depth to do, others are left alone.
+__global__ void __launch_bounds__(256) cap_factor_kernel(CapFactorArgs a, const int *only) {
+  if (only && !only[blockIdx.x]) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_info;
   const int p = blockIdx.x, node = a.node_base + p;
@@ -631,7 +634,17 @@ cudaError_t launch_cap_factor(const CapFactorArgs &a, cudaStream_t s) {
   const size_t bytes = (size_t)n2 * n2 * 8 + (size_t)n2 * 32 * 8 + (size_t)n2 * 4 + 16;
   cudaError_t e = set_smem(cap_factor_kernel, bytes);
   if (e != cudaSuccess) return e;
-  HODLR_LAUNCH(cap_factor_kernel, a.nnode, 256, bytes, s, a);
+  HODLR_LAUNCH(cap_factor_kernel, a.nnode, 256, bytes, s, a, nullptr);
+  return cudaGetLastError();
+}
+
+// The nodes with only[p] != 0, whatever their size.
+cudaError_t launch_cap_factor_marked(const CapFactorArgs &a, const int *only, cudaStream_t s) {
+  const int n2 = 2 * a.r;
+  const size_t bytes = (size_t)n2 * n2 * 8 + (size_t)n2 * 32 * 8 + (size_t)n2 * 4 + 16;
+  cudaError_t e = set_smem(cap_factor_kernel, bytes);
+  if (e != cudaSuccess) return e;
+  HODLR_LAUNCH(cap_factor_kernel, a.nnode, 256, bytes, s, a, only);
   return cudaGetLastError();
 }
 
@@ -908,6 +921,36 @@ cudaError_t launch_cap_apply(const CapApplyArgs &a, cudaStream_t s) {
   const int NP = MT * 32;
   const bool dw = a.sinv2 != nullptr;
   if (!dw && a.C <= 8) return launch_f64_thin_cap(a, s);
+  const char *no_tc = getenv("HODLR_NO_TCGEN05");
+  if (!dw && !a.trans && !a.eta32 && !(no_tc && no_tc[0] == '1')) {
+    // On the tensor cores, as two products over the nodes: the inverse's first r
+    // columns times s.T1, its last r times s.T0.  4096 nodes of rank 32 and 384
+    // columns take 2.4 ms so, 12 at the FP64 FMA rate.
+    UpdateArgs ua{};
+    ua.lda = n2;
+    ua.a_bstride = (long long)n2 * n2;
+    ua.ldb = a.r;
+    ua.b_s1 = 4 * a.tb_stride;
+    ua.b_s2 = 2 * a.tb_stride;
+    ua.scale = a.scale;
+    ua.C = a.eta;
+    ua.ldc = n2;
+    ua.c_bstride = (long long)n2 * a.C;
+    ua.M = n2;
+    ua.N = a.C;
+    ua.K = a.r;
+    ua.nbatch = a.nnode;
+    ua.alpha = 1.0;
+    ua.skip = a.skip;
+    for (int h = 0; h < 2; ++h) {
+      ua.A = a.sinv + ((long long)a.node_base * n2 + (long long)h * a.r) * n2;
+      ua.B = a.Tb + (h ? 0 : a.tb_stride);
+      ua.overwrite = h == 0;
+      const cudaError_t e = launch_update_nn<double>(ua, s);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  }
   const size_t es = dw ? sizeof(float2) : sizeof(double);
   const size_t bytes = (size_t)NP * NP * es + (size_t)NP * 32 * es;
   // enough CTAs to fill the GPU, each covering several column tiles of its node

@@ -311,7 +311,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
     double *Cr = c_ptr(w, jn), *Cn = Cr;
     if (t0 >= t1) jn = 0;
 #pragma unroll
-    for (int c = 0; c < kEpiCols; ++c) cv[c] = c < jn ? Cr[(long long)c * a.ldc] : 0.0;
+    for (int c = 0; c < kEpiCols; ++c) cv[c] = c < jn && !a.overwrite ? Cr[(long long)c * a.ldc] : 0.0;
     while (w.t < t1) {
       const int ti = w.t - t0, slot = ti & 1, rt = w.rt;
       w.next();
@@ -342,7 +342,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
         for (int c = 0; c < 2; ++c) {
           const int cc = c2 + c;
           if (cc < jn) Cr[(long long)cc * a.ldc] = fma(a.alpha, x[c], cv[cc]);
-          cv[cc] = cc < jn1 ? Cn[(long long)cc * a.ldc] : 0.0;
+          cv[cc] = cc < jn1 && !a.overwrite ? Cn[(long long)cc * a.ldc] : 0.0;
         }
       }
       Cr = Cn;

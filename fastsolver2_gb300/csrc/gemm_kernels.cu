@@ -779,13 +779,13 @@ cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st)
     if (update_tma_try(a, st, s, e)) return e;
   } else {
     cudaError_t e = cudaSuccess;
-    if (a.overwrite && (a.K > 4 || a.a_trans)) return cudaErrorInvalidValue;  // the others add to C
     // Up to 4 columns, or 4 inner values, the FP64 FMAs are few and every value
     // is read once by the thin kernels; from 5 on a 128 x 32 tile takes 6 us of an
     // SM on the tensor cores, and 8 columns 8 us on the FMA pipe (rank 32)
     if (!a.a_trans && a.K <= 4) return launch_f64_thin_outer(a, s);
-    if (!a.a_trans && a.N <= 4) return launch_f64_thin_update(a, s);
+    if (!a.a_trans && a.N <= 4 && !a.overwrite) return launch_f64_thin_update(a, s);
     if (!tensor_cores_off() && f64_update_tc_try(a, st, s, e)) return e;
+    if (a.overwrite) return cudaErrorInvalidValue;  // the others add to C
     if (!a.a_trans && a.N <= 8) return launch_f64_thin_update(a, s);
   }
   const int nrt = ceil_div(a.M, kUpdBM), nct = ceil_div(a.N, kUpdBN);

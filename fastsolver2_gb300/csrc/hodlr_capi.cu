@@ -142,6 +142,7 @@ struct hodlr_ctx {
   // application, their row scales and balances (null: FMA kernels only)
   unsigned char *Dimg = nullptr;
   int *Drow = nullptr, *Dbal = nullptr;
+  void *capw = nullptr;  // FP64 mode: workspace of the blocked capacitance factorisation (null: one CTA a node)
   bool factored = false;
   // workspaces
   double *Tbuf = nullptr, *Wbuf = nullptr, *eta = nullptr, *red = nullptr;
@@ -661,7 +662,7 @@ template <typename T> static int factor_sweep(hodlr_ctx *h, bool leaves_done = f
     cf.nnode = h->nodes(l);
     cf.node_base = h->node_base(l);
     cf.st = h->dst;
-    PHASE(h, HODLR_PHASE_CAPACITANCE, launch_cap_factor(cf, s));
+    PHASE(h, HODLR_PHASE_CAPACITANCE, sizeof(T) == 8 && h->capw ? launch_f64_cap_gj(cf, h->capw, s) : launch_cap_factor(cf, s));
     if (Cd > 0) {
       CKS(cap_apply(h, l, Cd, (long long)r * Ct, false, nullptr));
       UpdateArgs ua{};
@@ -1370,6 +1371,18 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
       if (ie == cudaSuccess) h->Drow = h->alloc<int>(f64_leaf_image_rows(m, h->nleaf), ie);
       if (ie == cudaSuccess) h->Dbal = h->alloc<int>((size_t)n, ie);
       if (ie == cudaSuccess) h->Dimg = img;
+    }
+    (void)cudaGetLastError();
+  }
+  if (!h->mixed && L > 0 && !(no_tc64 && no_tc64[0] == '1')) {
+    int most = 0;
+    for (int l = 0; l < L; ++l) most = std::max(most, h->nodes(l));
+    const size_t bytes = f64_cap_gj_scratch(r, most);
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) == cudaSuccess && bytes <= avail / 4) {
+      cudaError_t ie = cudaSuccess;
+      h->capw = h->alloc<unsigned char>(bytes, ie);
+      if (ie != cudaSuccess) h->capw = nullptr;
     }
     (void)cudaGetLastError();
   }

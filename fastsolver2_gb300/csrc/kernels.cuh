@@ -118,7 +118,9 @@ struct UpdateArgs {
   int M, N, K, nbatch;
   double alpha;
   const int *skip;
-  int overwrite;  // FP64, K <= 4: C_b = instead of += (its old values are not read)
+  // C_b = instead of += (its old values are not read): FP64 with K <= 4, or on
+  // the tensor cores
+  int overwrite;
 };
 // f64_thin.cu: the FP64 steps for up to 8 columns (update, reduction, leaf and
 // capacitance application), and updates of an inner dimension up to 4
@@ -163,7 +165,7 @@ cudaError_t launch_f64_leaf_tc(const unsigned char *img, const int *rows, const 
                                DevStatus *st, cudaStream_t s);
 
 // Dinv = D^-1 of leaves of 64, 128 or 256 rows by blocked Gauss-Jordan, the
-// products on the tensor cores (f64_leaf_gj.cu; no LU factors).  A: workspace
+// products on the tensor cores (f64_gj.cu; no LU factors).  A: workspace
 // [nleaf][m][m], ipiv: workspace [nleaf][m]; scratch: f64_leaf_gj_scratch bytes,
 // 8-byte aligned.
 size_t f64_leaf_gj_scratch(int m, int nleaf);
@@ -185,6 +187,11 @@ struct CapFactorArgs {
   DevStatus *st;
 };
 cudaError_t launch_cap_factor(const CapFactorArgs &a, cudaStream_t s);
+// The same in FP64 (LU, pivots and Sinv) by blocked Gauss-Jordan, the products
+// on the tensor cores (f64_gj.cu).  scratch: f64_cap_gj_scratch bytes, 8-byte
+// aligned.
+size_t f64_cap_gj_scratch(int r, int nnode);
+cudaError_t launch_f64_cap_gj(const CapFactorArgs &a, void *scratch, cudaStream_t s);
 
 // eta_p = op(Sinv_p) RHS_p (2r x C per node, ld 2r) with RHS_p built from the
 // T blocks (forward: [s.T1; s.T0], transposed: [T0; T1]).  Double-word

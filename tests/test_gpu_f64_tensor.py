@@ -252,3 +252,71 @@ def test_singular_leaf_is_refused(lib, m, kind):
     with pytest.raises(lib.HodlrError) as e:
         factored_leaves(lib, D, np.ones((2 * m, 1)))
     assert e.value.code == lib.HODLR_ERR_SINGULAR_LEAF and "index 1" in str(e.value)
+
+
+# padded sizes 32, 64 and 128 and their edges: 2r at, below and above a panel
+@pytest.mark.parametrize("r", [1, 8, 15, 16, 17, 31, 32, 33, 48, 64])
+def test_capacitance_factors_of_a_solver(lib, r):
+    """The LU factors, pivots and solutions of the capacitance systems of a
+    two-level solver with identity leaves: S = [I, s V1^T U1; s V0^T U0, I] of the
+    bottom nodes, P S = L U, and x against a dense solve.  Bounds: the standard
+    componentwise bound of a factorisation of order n, 2 n 2^-53 |L| |U|, and 4 n
+    2^-53 cond^2 for the inverses, on the whole matrix."""
+    rng = np.random.default_rng(r)
+    m, L = 128, 2
+    n = m << L
+    D = np.stack([np.eye(m)] * (1 << L))
+    Us, Vs = ([rng.standard_normal((n, r)) / np.sqrt(m) for _ in range(L)] for _ in range(2))
+    s = lib.Solver(n, m, L, r, nrhs_max=12)
+    s.set_leaf_blocks(torch.from_numpy(D).cuda().reshape(-1), ld=m, leaf_stride=m * m)
+    for l in range(L):
+        s.set_lowrank(l, col(Us[l]), col(Vs[l]))
+    s.factor()
+    n2 = 2 * r
+    lu = torch.zeros(3 * n2 * n2, dtype=torch.float64, device="cuda")
+    piv = torch.zeros(3 * n2, dtype=torch.int32, device="cuda")
+    s.get_factors(cap_lu=lu, cap_ipiv=piv)
+    lu, piv = lu.cpu().numpy().reshape(3, n2, n2).transpose(0, 2, 1), piv.cpu().numpy().reshape(3, n2)
+    # one level of the recursion by node numbering: the two nodes of either end of the list
+    found = 0
+    for q in range(2):
+        c0, c1 = slice(2 * q * m, (2 * q + 1) * m), slice((2 * q + 1) * m, (2 * q + 2) * m)
+        S = np.eye(n2)
+        S[:r, r:], S[r:, :r] = Vs[L - 1][c1].T @ Us[L - 1][c1], Vs[L - 1][c0].T @ Us[L - 1][c0]
+        for k in range(3):
+            P, Lf, R = S.copy(), np.tril(lu[k], -1) + np.eye(n2), np.triu(lu[k])
+            for i, p in enumerate(piv[k]):
+                P[[i, p - 1]] = P[[p - 1, i]]
+            # S itself is formed from sums of m products: m 2^-53 |V|^T |U| more
+            slack = np.pad(np.zeros((r, r)), (0, r))
+            slack[:r, r:], slack[r:, :r] = (np.abs(Vs[L - 1][c]).T @ np.abs(Us[L - 1][c]) for c in (c1, c0))
+            bound = 2 * n2 * HALF_ULP * (np.abs(Lf) @ np.abs(R)) + m * HALF_ULP * slack.max()
+            found += (np.abs(P - Lf @ R) <= bound).all()
+    assert found == 2
+    A = np.eye(n)
+    for l in range(L):
+        h = n >> (l + 1)
+        for p in range(1 << l):
+            c0, c1 = slice(2 * p * h, (2 * p + 1) * h), slice((2 * p + 1) * h, (2 * p + 2) * h)
+            A[c0, c1], A[c1, c0] = Us[l][c0] @ Vs[l][c1].T, Us[l][c1] @ Vs[l][c0].T
+    B = rng.standard_normal((n, 12))
+    b = col(B)
+    s.solve(b)
+    exact = np.linalg.solve(A, B)
+    err = np.linalg.norm(b.cpu().numpy() - exact) / np.linalg.norm(exact)
+    assert err <= 4 * n * HALF_ULP * np.linalg.cond(A) ** 2
+
+
+def test_singular_capacitance_is_refused(lib):
+    """A = [I, e e^T; e e^T, I] on one node: S is exactly singular."""
+    m, r = 128, 20
+    s = lib.Solver(2 * m, m, 1, r)
+    D = np.stack([np.eye(m)] * 2)
+    U = np.zeros((2 * m, r))
+    for q in range(r):
+        U[q, q] = U[m + q, q] = 1.0
+    s.set_leaf_blocks(torch.from_numpy(D).cuda().reshape(-1), ld=m, leaf_stride=m * m)
+    s.set_lowrank(0, col(U), col(U))
+    with pytest.raises(lib.HodlrError) as e:
+        s.factor()
+    assert e.value.code == lib.HODLR_ERR_SINGULAR_CAPACITANCE
