@@ -85,7 +85,7 @@ __device__ __forceinline__ double newton_rcp(double x) {
 template <int M, bool LU> __host__ __device__ constexpr int gj_threads() { return LU ? 2 * M : M + kNb; }
 template <int M, bool LU>
 __global__ void __launch_bounds__(gj_threads<M, LU>())
-gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, const unsigned *big, int *again, LuOut out) {
+gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, int nc, const unsigned *big, int *again, LuOut out) {
   constexpr int NW = M / 32;  // warps with rows of the block; the next has the identity's
   __shared__ double sU[2][NW][kNb], sRcp[2][NW], sL[kNb][kNb];
   __shared__ uint4 sBest[2][NW];  // |a| (high, low word), position, row of each warp's candidate
@@ -97,8 +97,10 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, const unsign
   const int orig = real ? (k0 ? perm[blk * M + tid] : tid) : 0;  // the row of D
   const unsigned *bl = big + blk * 2 * M;                         // largest |D| of its rows, then its columns
   const unsigned brow = real ? bl[orig] : 0;
-  bool open = real && tid >= k0;  // may still become a pivot row
-  bool pivot_row = false;
+  // the identity's rows and columns that pad the block are their own pivots: no
+  // steps for the panel's columns from nc on
+  bool pivot_row = LU && real && tid >= k0 + nc && tid < k0 + kNb;
+  bool open = real && tid >= k0 && !pivot_row;  // may still become a pivot row
   double a[kNb];
 #pragma unroll
   for (int c = 0; c < kNb; ++c) a[c] = real ? Al[tid + (long long)(k0 + c) * M] : (c == lane ? 1.0 : 0.0);
@@ -137,6 +139,7 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, const unsign
   __syncthreads();
 #pragma unroll
   for (int c = 0; c < kNb; ++c) {
+    if (LU && c >= nc) continue;
     const int buf = c & 1;
     uint4 best = sBest[buf][0];
     int bw = 0;
@@ -170,7 +173,7 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, const unsign
       a[c] = l;
       if (c + 1 < kNb) a[c + 1] -= l * u[c + 1];
     }
-    if (c + 1 < kNb) {
+    if (c + 1 < (LU ? nc : kNb)) {
       cand = candidate(a[c + 1]);
       rc = newton_rcp(a[c + 1]);
       if (row) {
@@ -227,6 +230,7 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, const unsign
       for (int c = 0; c < kNb; ++c) a[c] = Rj[c];
 #pragma unroll
       for (int c = 0; c < kNb; ++c) {
+        if (c >= nc) continue;
 #pragma unroll
         for (int t = c + 1; t < kNb; ++t) a[t] -= sL[t][c] * a[c];
       }
@@ -239,9 +243,11 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, const unsign
     // times L11^-1 from the right: W, and the panel's new columns (the identity's
     // rows, now D^-1, are the pivot rows')
 #pragma unroll
-    for (int t = kNb - 1; t > 0; --t)
+    for (int t = kNb - 1; t > 0; --t) {
+      if (LU && t >= nc) continue;
 #pragma unroll
       for (int c = 0; c < t; ++c) a[c] -= a[t] * sL[t][c];
+    }
     double *Wl = W + blk * M * kNb;
     const int row = real ? pos : k0 + lane;
 #pragma unroll
@@ -335,7 +341,8 @@ template <bool LU>
 static cudaError_t gj_blocks(int m, int n, int count, double *A, double *W, double *R, int *perm, const unsigned *big,
                              int *again, const LuOut &out, DevStatus *st, cudaStream_t s) {
 #define HODLR_GJ(MV)                                                                                            \
-  HODLR_LAUNCH((gj_panel_kernel<MV, LU>), count, (gj_threads<MV, LU>()), 0, s, A, W, R, perm, k0, big, again, out)
+  HODLR_LAUNCH((gj_panel_kernel<MV, LU>), count, (gj_threads<MV, LU>()), 0, s, A, W, R, perm, k0, std::min(kNb, n - k0), big, again, \
+               out)
   for (int k0 = 0; k0 < n; k0 += kNb) {
     if (m == 64) {
       HODLR_GJ(64);
@@ -398,16 +405,16 @@ __global__ void __launch_bounds__(256) cap_gj_build_kernel(CapFactorArgs a, int 
                                                            int *again) {
   __shared__ unsigned srow[128], scol[128];
   const int p = blockIdx.x, tid = threadIdx.x, r = a.r, n2 = 2 * r;
-  const double *T0 = a.Tb + (long long)(2 * p) * a.tb_stride + (long long)a.ucol * r;
-  const double *T1 = a.Tb + (long long)(2 * p + 1) * a.tb_stride + (long long)a.ucol * r;
+  const long long o0 = (long long)(2 * p) * a.tb_stride + (long long)a.ucol * r, o1 = o0 + a.tb_stride;
+  auto T = [&](long long off) -> double { return a.Tb32 ? (double)a.Tb32[off] : a.Tb[off]; };
   if (tid < m) srow[tid] = scol[tid] = 0;
   __syncthreads();
   unsigned mx = 0;
   for (int e = tid; e < m * m; e += 256) {
     const int i = e % m, j = e / m;
     double v = i == j ? 1.0 : 0.0;
-    if (i >= r && i < n2 && j < r) v = (a.scale ? a.scale[i - r] : 1.0) * T0[i - r + (long long)j * r];
-    if (i < r && j >= r && j < n2) v = (a.scale ? a.scale[i] : 1.0) * T1[i + (long long)(j - r) * r];
+    if (i >= r && i < n2 && j < r) v = (a.scale ? a.scale[i - r] : 1.0) * T(o0 + i - r + (long long)j * r);
+    if (i < r && j >= r && j < n2) v = (a.scale ? a.scale[i] : 1.0) * T(o1 + i + (long long)(j - r) * r);
     A[(long long)p * m * m + e] = v;
     const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu;
     mx = max(mx, h);
@@ -423,13 +430,19 @@ __global__ void __launch_bounds__(256) cap_gj_build_kernel(CapFactorArgs a, int 
   if (tid == 0) again[p] = 0;
 }
 
-// Sinv's columns from the inverse of the interchanged rows.
+// Sinv's columns from the inverse of the interchanged rows (FP32 if sinv32).
 __global__ void __launch_bounds__(256) cap_gj_columns_kernel(const double *__restrict__ A, const int *__restrict__ perm,
-                                                             int m, int n2, double *sinv) {
+                                                             int m, int n2, double *sinv, float *sinv32) {
   const long long p = blockIdx.x;
   for (int e = threadIdx.x; e < n2 * n2; e += 256) {
     const int i = e % n2, j = e / n2, c = perm[p * m + j];
-    if (c < n2) sinv[p * n2 * n2 + i + (long long)c * n2] = A[p * m * m + i + (long long)j * m];
+    const double v = A[p * m * m + i + (long long)j * m];
+    const long long o = p * n2 * n2 + i + (long long)c * n2;
+    if (c >= n2) continue;
+    if (sinv32)
+      sinv32[o] = f64_to_f32_rn(v);
+    else
+      sinv[o] = v;
   }
 }
 
@@ -452,7 +465,9 @@ cudaError_t launch_f64_cap_gj(const CapFactorArgs &a, void *scratch, cudaStream_
   HODLR_LAUNCH(cap_gj_build_kernel, a.nnode, 256, 0, s, a, m, A, big, again);
   cudaError_t e = gj_blocks<true>(m, n2, a.nnode, A, W, R, perm, big, again, out, a.st, s);
   if (e != cudaSuccess) return e;
-  HODLR_LAUNCH(cap_gj_columns_kernel, a.nnode, 256, 0, s, A, perm, m, n2, a.sinv + (long long)a.node_base * n2 * n2);
+  const long long base = (long long)a.node_base * n2 * n2;
+  HODLR_LAUNCH(cap_gj_columns_kernel, a.nnode, 256, 0, s, A, perm, m, n2, a.sinv ? a.sinv + base : nullptr,
+               a.sinv32 ? a.sinv32 + base : nullptr);
   return launch_cap_factor_marked(a, again, s);
 }
 

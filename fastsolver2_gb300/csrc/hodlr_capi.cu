@@ -142,7 +142,11 @@ struct hodlr_ctx {
   // application, their row scales and balances (null: FMA kernels only)
   unsigned char *Dimg = nullptr;
   int *Drow = nullptr, *Dbal = nullptr;
-  void *capw = nullptr;  // FP64 mode: workspace of the blocked capacitance factorisation (null: one CTA a node)
+  // workspace of the blocked capacitance factorisation (null: one CTA a node):
+  // FP64 mode, and mixed mode for ranks above 32 (a 128 x 128 system takes 0.95
+  // ms in one CTA and 0.45 in blocks; up to 64 x 64 one CTA is the faster one,
+  // 0.13 to 0.19 against 0.23)
+  void *capw = nullptr;
   bool factored = false;
   // workspaces
   double *Tbuf = nullptr, *Wbuf = nullptr, *eta = nullptr, *red = nullptr;
@@ -662,7 +666,7 @@ template <typename T> static int factor_sweep(hodlr_ctx *h, bool leaves_done = f
     cf.nnode = h->nodes(l);
     cf.node_base = h->node_base(l);
     cf.st = h->dst;
-    PHASE(h, HODLR_PHASE_CAPACITANCE, sizeof(T) == 8 && h->capw ? launch_f64_cap_gj(cf, h->capw, s) : launch_cap_factor(cf, s));
+    PHASE(h, HODLR_PHASE_CAPACITANCE, h->capw ? launch_f64_cap_gj(cf, h->capw, s) : launch_cap_factor(cf, s));
     if (Cd > 0) {
       CKS(cap_apply(h, l, Cd, (long long)r * Ct, false, nullptr));
       UpdateArgs ua{};
@@ -1374,7 +1378,7 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
     }
     (void)cudaGetLastError();
   }
-  if (!h->mixed && L > 0 && !(no_tc64 && no_tc64[0] == '1')) {
+  if ((!h->mixed || r > 32) && L > 0 && !(no_tc64 && no_tc64[0] == '1')) {
     int most = 0;
     for (int l = 0; l < L; ++l) most = std::max(most, h->nodes(l));
     const size_t bytes = f64_cap_gj_scratch(r, most);
