@@ -27,6 +27,8 @@
 #include <tuple>
 #include <vector>
 
+#include <cuda.h>
+
 #include "kernels.cuh"
 #include "ozaki.cuh"
 #include "resid_emul.cuh"
@@ -1479,13 +1481,101 @@ int hodlr_set_stream(hodlr_handle h, void *stream) {
   return HODLR_OK;
 }
 
+}  // extern "C"
+
+// Whether rows x cols doubles at p (leading dimension ld) lie in one device
+// allocation of the current device: then a kernel may read them; every other
+// source -- host and managed memory, another device's, a range the copy call
+// will refuse -- goes through cudaMemcpy.
+static bool on_device(const double *p, long long ld, long long rows, long long cols) {
+  typedef CUresult (*RangeFn)(CUdeviceptr *, size_t *, CUdeviceptr);
+  static const RangeFn range = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 3020, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    (void)cudaGetLastError();
+    return reinterpret_cast<RangeFn>(f);
+  }();
+  int dev = 0;
+  cudaPointerAttributes a{};
+  const bool ok = range && cudaGetDevice(&dev) == cudaSuccess && cudaPointerGetAttributes(&a, p) == cudaSuccess &&
+                  a.type == cudaMemoryTypeDevice && a.device == dev;
+  (void)cudaGetLastError();
+  if (!ok || rows < 1 || cols < 1 || ((uintptr_t)p & 7)) return false;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  if (range(&base, &size, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return false;
+  const unsigned long long need = sizeof(double) * ((unsigned long long)(cols - 1) * ld + rows);
+  return (unsigned long long)((uintptr_t)p - (uintptr_t)base) + need <= size;
+}
+
+// Leaf blocks [leaf0, leaf0 + nl) from device memory: the copy, with the digits
+// of the tensor-core residual in the same pass.  *done: nothing is left to prepare
+// from them but the leaf factorisation.
+static int copy_leaves_device(hodlr_ctx *h, const double *D, int64_t ld, int64_t leaf_stride, long long leaf0,
+                              long long nl, bool *done) {
+  const long long m = h->m, mm = m * m;
+  *done = false;
+  if (h->oz) {
+    const cudaError_t e = launch_set_rows(D, m, leaf_stride, ld, h->D + leaf0 * mm, mm, m, nl * m, (int)m,
+                                          h->Dsl + leaf0 * mm, h->n * m, h->Dexp + leaf0 * m, h->st);
+    if (e == cudaSuccess) {
+      if (h->emulated) h->dw_stale = true;
+      *done = true;
+      return HODLR_OK;
+    }
+    if (e != cudaErrorNotSupported) CK(e);
+  }
+  if (ld == m && leaf_stride == mm)
+    CK(launch_copy2d(D, mm * nl, h->D + leaf0 * mm, mm * nl, mm * nl, 1, h->st));
+  else
+    CK(launch_pack_leaves(D, ld, leaf_stride, h->D + leaf0 * mm, (int)m, (int)nl, h->st));
+  return HODLR_OK;
+}
+
+// The same for the rows [row0, row0 + rows) of level l's U and V.
+static int copy_level_device(hodlr_ctx *h, int l, long long row0, long long rows, const double *U, int64_t ldu,
+                             const double *V, int64_t ldv, bool *done_u, bool *done_v) {
+  const long long n = h->n, r = h->r, L = h->L;
+  double *Ud = h->Ulev(l) + row0, *Vd = h->Vlev(l) + row0;
+  *done_u = *done_v = false;
+  if (h->oz) {
+    cudaError_t e = launch_set_rows(U, rows, 0, ldu, Ud, 0, n, rows, (int)r, h->Usl + l * n * r + row0 * r, L * n * r,
+                                    h->Uexp + l * n + row0, h->st);
+    if (e != cudaErrorNotSupported) CK(e);
+    *done_u = e == cudaSuccess;
+    e = launch_set_cols(V, ldv, Vd, h->V32 + l * n * r + row0, n, rows, (int)r, h->Vsl + l * r * n + row0, L * n * r,
+                        h->Vexp + l * (n / kOzChunk) * r + (row0 / kOzChunk) * r, h->st);
+    if (e != cudaErrorNotSupported) CK(e);
+    *done_v = e == cudaSuccess;
+    if (h->emulated && (*done_u || *done_v)) h->dw_stale = true;
+  }
+  if (!*done_u) CK(launch_copy2d(U, ldu, Ud, n, rows, (int)r, h->st));
+  if (!*done_v) CK(launch_copy2d(V, ldv, Vd, n, rows, (int)r, h->st));
+  return HODLR_OK;
+}
+
+// Rows a leaf array of ld and leaf_stride spans, as one column-major matrix of m
+// columns or as blocks one after another.
+static bool leaves_on_device(const double *D, long long ld, long long leaf_stride, long long m, long long nl) {
+  if (leaf_stride < 0) return false;
+  return on_device(D, 1, leaf_stride * (nl - 1) + ld * (m - 1) + m, 1);
+}
+
+extern "C" {
+
 int hodlr_set_leaf_blocks(hodlr_handle h, const double *D, int64_t ld, int64_t leaf_stride) {
   if (!h || !D) return set_err(HODLR_ERR_INVALID_ARG, "null argument");
   if (ld < h->m) return set_err(HODLR_ERR_INVALID_ARG, "ld < leaf size");
   const int m = h->m;
   const long long mm = (long long)m * m;
   CKS(wait_prepared(h, 0));
-  if (ld == m && leaf_stride == mm) {
+  bool prepared = false;
+  if (leaves_on_device(D, ld, leaf_stride, m, h->nleaf)) {
+    CKS(copy_leaves_device(h, D, ld, leaf_stride, 0, h->nleaf, &prepared));
+  } else if (ld == m && leaf_stride == mm) {
     CK(cudaMemcpyAsync(h->D, D, sizeof(double) * mm * h->nleaf, cudaMemcpyDefault, h->st));
   } else {
     // column j of every leaf in one strided copy (host or device source)
@@ -1498,7 +1588,7 @@ int hodlr_set_leaf_blocks(hodlr_handle h, const double *D, int64_t ld, int64_t l
   h->factored = false;
   h->leaves_prefactored = false;
   return prepare_input(h, 0, [&](cudaStream_t ps) -> int {
-    CKS(prepare_leaves(h, 0, -1, ps));
+    if (!prepared) CKS(prepare_leaves(h, 0, -1, ps));
     if (h->mixed && ps != h->st) {
       // the leaf LU (+ inverses) depends on the leaf blocks alone: it runs on
       // the side stream while the low-rank inputs are still being copied
@@ -1524,12 +1614,17 @@ int hodlr_set_lowrank(hodlr_handle h, int level, const double *U, int64_t ldu, c
     if (cudaPointerGetAttributes(&a, V) == cudaSuccess && a.type == cudaMemoryTypeHost) defer = true;
     (void)cudaGetLastError();
   }
-  // plain (2-D) copies: the sources may be device or host memory
-  CK(cudaMemcpy2DAsync(h->Ulev(level), sizeof(double) * h->n, U, sizeof(double) * ldu, sizeof(double) * h->n,
-                       h->r, cudaMemcpyDefault, h->st));
-  if (!defer)
-    CK(cudaMemcpy2DAsync(h->Vlev(level), sizeof(double) * h->n, V, sizeof(double) * ldv, sizeof(double) * h->n,
+  bool done_u = false, done_v = false;
+  if (!defer && on_device(U, ldu, h->n, h->r) && on_device(V, ldv, h->n, h->r)) {
+    CKS(copy_level_device(h, level, 0, h->n, U, ldu, V, ldv, &done_u, &done_v));
+  } else {
+    // plain (2-D) copies: the sources may be device or host memory
+    CK(cudaMemcpy2DAsync(h->Ulev(level), sizeof(double) * h->n, U, sizeof(double) * ldu, sizeof(double) * h->n,
                          h->r, cudaMemcpyDefault, h->st));
+    if (!defer)
+      CK(cudaMemcpy2DAsync(h->Vlev(level), sizeof(double) * h->n, V, sizeof(double) * ldv, sizeof(double) * h->n,
+                           h->r, cudaMemcpyDefault, h->st));
+  }
   h->vsrc[level] = defer ? V : nullptr;
   h->vsrc_ld[level] = ldv;
   if (s)
@@ -1540,7 +1635,11 @@ int hodlr_set_lowrank(hodlr_handle h, int level, const double *U, int64_t ldu, c
   h->factored = false;
   if (defer)
     return prepare_input(h, 1 + level, [&](cudaStream_t ps) { return prepare_level_u(h, level, 0, -1, ps); });
-  return prepare_input(h, 1 + level, [&](cudaStream_t ps) { return prepare_level(h, level, 0, -1, ps); });
+  if (done_u && done_v) return HODLR_OK;  // nothing left for the side stream
+  return prepare_input(h, 1 + level, [&](cudaStream_t ps) -> int {
+    if (!done_u) CKS(prepare_level_u(h, level, 0, -1, ps));
+    return done_v ? HODLR_OK : prepare_level_v(h, level, 0, -1, ps);
+  });
 }
 
 int hodlr_factor(hodlr_handle h) {
@@ -2593,14 +2692,17 @@ int hodlr_batch_set_leaf_blocks(hodlr_batch b, int i, const double *D, int64_t l
   if (ld < m) return set_err(HODLR_ERR_INVALID_ARG, "batch: ld < leaf size");
   const long long mm = (long long)m * m, leaf0 = mb.row_off / m, nl = sy.n / m;
   double *dst = h->D + leaf0 * mm;
-  if (ld == m && leaf_stride == mm) {
+  bool prepared = false;
+  if (leaves_on_device(D, ld, leaf_stride, m, nl)) {
+    CKS(copy_leaves_device(h, D, ld, leaf_stride, leaf0, nl, &prepared));
+  } else if (ld == m && leaf_stride == mm) {
     CK(cudaMemcpyAsync(dst, D, sizeof(double) * mm * nl, cudaMemcpyDefault, h->st));
   } else {
     for (int j = 0; j < m; ++j)
       CK(cudaMemcpy2DAsync(dst + (long long)j * m, sizeof(double) * mm, D + (long long)j * ld,
                            sizeof(double) * leaf_stride, sizeof(double) * m, nl, cudaMemcpyDefault, h->st));
   }
-  CKS(prepare_leaves(h, leaf0, nl));
+  if (!prepared) CKS(prepare_leaves(h, leaf0, nl));
   mb.has_D = true;
   b->factored = false;
   CK(cudaStreamSynchronize(h->st));
@@ -2617,15 +2719,22 @@ int hodlr_batch_set_lowrank(hodlr_batch b, int i, int level, const double *U, in
   if (ldu < sy.n || ldv < sy.n) return set_err(HODLR_ERR_INVALID_ARG, "batch: ld < n");
   const int slot = mb.slot0 + level, r = h->r;
   double *Ud = h->Ulev(slot) + mb.row_off, *Vd = h->Vlev(slot) + mb.row_off;
-  CK(cudaMemcpy2DAsync(Ud, sizeof(double) * h->n, U, sizeof(double) * ldu, sizeof(double) * sy.n, r,
-                       cudaMemcpyDefault, h->st));
-  CK(cudaMemcpy2DAsync(Vd, sizeof(double) * h->n, V, sizeof(double) * ldv, sizeof(double) * sy.n, r,
-                       cudaMemcpyDefault, h->st));
+  bool done_u = false, done_v = false;
+  if (on_device(U, ldu, sy.n, r) && on_device(V, ldv, sy.n, r)) {
+    CKS(copy_level_device(h, slot, mb.row_off, sy.n, U, ldu, V, ldv, &done_u, &done_v));
+  } else {
+    CK(cudaMemcpy2DAsync(Ud, sizeof(double) * h->n, U, sizeof(double) * ldu, sizeof(double) * sy.n, r,
+                         cudaMemcpyDefault, h->st));
+    CK(cudaMemcpy2DAsync(Vd, sizeof(double) * h->n, V, sizeof(double) * ldv, sizeof(double) * sy.n, r,
+                         cudaMemcpyDefault, h->st));
+  }
   if (s) {
     CK(cudaMemcpyAsync(h->sfold, s, sizeof(double) * r, cudaMemcpyDefault, h->st));
     CK(launch_scale_cols(Vd, h->n, sy.n, r, h->sfold, h->st));
+    done_v = false;  // its derived copies are of the scaled V
   }
-  CKS(prepare_level(h, slot, mb.row_off, sy.n));
+  if (!done_u) CKS(prepare_level_u(h, slot, mb.row_off, sy.n));
+  if (!done_v) CKS(prepare_level_v(h, slot, mb.row_off, sy.n));
   mb.has_level[level] = 1;
   b->factored = false;
   CK(cudaStreamSynchronize(h->st));

@@ -1,6 +1,8 @@
 // Launchers of the HODLR kernels (host side).  Every launcher enqueues on
 // the given stream and returns the launch error (if any).
 #pragma once
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace hodlr {
@@ -220,6 +222,19 @@ cudaError_t launch_convert(const Tin *X, long long ldx, Tout *Y, long long ldy, 
 // Pack leaf blocks (leaf i at D + i*stride, ld) into [nleaf][m][m].
 cudaError_t launch_pack_leaves(const double *D, long long ld, long long stride, double *out, int m,
                                int nleaf, cudaStream_t s);
+// Inputs from device memory (set_inputs.cu): a plain column-major copy; the copy
+// of row-scaled inputs (rows in blocks of rpb at bstride / dbstride) with their
+// digits and exponents (out + i cols + q, slice stride sstride); the copy of V
+// with its FP32 form and column-scaled digits.  The latter two return
+// cudaErrorNotSupported, with nothing launched, for sizes or alignments they do
+// not take.
+cudaError_t launch_copy2d(const double *src, long long lds, double *dst, long long ldd, long long rows, int cols,
+                          cudaStream_t s);
+cudaError_t launch_set_rows(const double *src, long long rpb, long long bstride, long long ld, double *dst,
+                            long long dbstride, long long ldd, long long rows, int cols, __nv_bfloat16 *out,
+                            long long sstride, int *exps, cudaStream_t s);
+cudaError_t launch_set_cols(const double *src, long long lds, double *dst, float *dst32, long long ldd, long long n,
+                            int c, __nv_bfloat16 *out, long long sstride, int *exps, cudaStream_t s);
 // Inverse of launch_pack_leaves: [nleaf][m][m] (type T) into leaf i at
 // out + i*stride (FP64, ld).
 template <typename T>

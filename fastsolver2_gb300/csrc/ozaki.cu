@@ -18,40 +18,6 @@
 
 namespace hodlr {
 
-// ------------------------------------------------------------------ digits
-// All on the integer pipes (GB300 issues FP64 at 1/58 of the FP32 rate):
-// magnitudes compare as their bit patterns, and a value's 49-bit fixed-point
-// image F = trunc(|a| 2^(49-E)) is its 53-bit significand shifted right by
-// E - e + 3 (e its unbiased exponent); the digits are F's 7-bit groups.
-__device__ __forceinline__ unsigned long long abs_bits(double v) {
-  return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-}
-
-// E with max|a| / 2^E in [0.5, 1) from the largest magnitude's bit pattern (0 for zero)
-__device__ __forceinline__ int oz_exponent_bits(unsigned long long maxbits) {
-  if (maxbits == 0) return 0;
-  const int ef = (int)(maxbits >> 52);
-  if (ef == 0) return -1010 - __clzll((long long)maxbits);  // subnormal: top bit p = 63 - clz, E = p - 1073
-  return ef - 1022;
-}
-
-template <typename Store>
-__device__ __forceinline__ void oz_digits(double v, int E, Store store) {
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
-  const int ef = (int)((bits >> 52) & 0x7ff);
-  const unsigned long long frac = bits & 0xfffffffffffffull;
-  const unsigned long long M = ef ? (frac | (1ull << 52)) : frac;  // |v| = M 2^(e - 52)
-  const int e = ef ? ef - 1023 : -1022;
-  const int sh = E - e + 3;  // >= 4 for normal v; a subnormal group may need a left shift
-  const unsigned long long F = (M == 0 || sh >= 64) ? 0ull : (sh >= 0 ? (M >> sh) : (M << -sh));
-  const bool neg = (bits >> 63) != 0;
-#pragma unroll
-  for (int s = 0; s < kOzSlices; ++s) {
-    const int d = (int)((F >> (42 - 7 * s)) & 127ull);
-    store(s, __int2bfloat16_rn(neg ? -d : d));
-  }
-}
-
 __global__ void oz_slice_rows_kernel(const double *A, long long rpb, long long bstride, long long si, long long sq,
                                      long long rows, int cols, __nv_bfloat16 *out, long long ld_out,
                                      long long sstride, int *exps) {
@@ -87,12 +53,10 @@ __global__ void oz_slice_rows8_kernel(const double *A, long long rpb, long long 
     double v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = row[(q0 + u) * sq];
-    __align__(16) __nv_bfloat16 d[kOzSlices][8];
+    uint4 d[kOzSlices];
+    oz_digits8(v, E, d);
 #pragma unroll
-    for (int u = 0; u < 8; ++u) oz_digits(v[u], E, [&](int sl, __nv_bfloat16 x) { d[sl][u] = x; });
-#pragma unroll
-    for (int sl = 0; sl < kOzSlices; ++sl)
-      *reinterpret_cast<uint4 *>(o + sl * sstride + q0) = *reinterpret_cast<const uint4 *>(d[sl]);
+    for (int sl = 0; sl < kOzSlices; ++sl) *reinterpret_cast<uint4 *>(o + sl * sstride + q0) = d[sl];
   }
 }
 
@@ -191,13 +155,11 @@ __global__ void oz_slice_cols8_kernel(const double *X, long long ldx, long long 
   for (int o = 4; o; o >>= 1) mb = max(mb, __shfl_xor_sync(gmask, mb, o));
   const int E = oz_exponent_bits(mb);
   if (sub == 0) exps[ch * c + j] = E;
-  __align__(16) __nv_bfloat16 d[kOzSlices][8];
-#pragma unroll
-  for (int u = 0; u < 8; ++u) oz_digits(v[u], E, [&](int sl, __nv_bfloat16 x) { d[sl][u] = x; });
+  uint4 d[kOzSlices];
+  oz_digits8(v, E, d);
   __nv_bfloat16 *o = out + j * ld_out + i0;
 #pragma unroll
-  for (int sl = 0; sl < kOzSlices; ++sl)
-    *reinterpret_cast<uint4 *>(o + sl * sstride) = *reinterpret_cast<const uint4 *>(d[sl]);
+  for (int sl = 0; sl < kOzSlices; ++sl) *reinterpret_cast<uint4 *>(o + sl * sstride) = d[sl];
 }
 
 cudaError_t launch_oz_slice_cols(const double *X, long long ldx, long long n, int c, __nv_bfloat16 *out,

@@ -26,6 +26,75 @@ namespace hodlr {
 constexpr int kOzSlices = 7;   // digits per operand (49 bits)
 constexpr int kOzChunk = 64;   // rows per exponent group of the column-scaled operands
 
+#ifdef __CUDACC__
+// ------------------------------------------------------------------ digits
+// All on the integer pipes (GB300 issues FP64 at 1/58 of the FP32 rate):
+// magnitudes compare as their bit patterns, and a value's 49-bit fixed-point
+// image F = trunc(|a| 2^(49-E)) is its 53-bit significand shifted right by
+// E - e + 3 (e its unbiased exponent); the digits are F's 7-bit groups.
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+
+// E with max|a| / 2^E in [0.5, 1) from the largest magnitude's bit pattern (0 for zero)
+__device__ __forceinline__ int oz_exponent_bits(unsigned long long maxbits) {
+  if (maxbits == 0) return 0;
+  const int ef = (int)(maxbits >> 52);
+  if (ef == 0) return -1010 - __clzll((long long)maxbits);  // subnormal: top bit p = 63 - clz, E = p - 1073
+  return ef - 1022;
+}
+
+// F of a value and its sign (1: negative).
+__device__ __forceinline__ unsigned long long oz_fixed(double v, int E, unsigned &neg) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+  const int ef = (int)((bits >> 52) & 0x7ff);
+  const unsigned long long frac = bits & 0xfffffffffffffull;
+  const unsigned long long M = ef ? (frac | (1ull << 52)) : frac;  // |v| = M 2^(e - 52)
+  const int e = ef ? ef - 1023 : -1022;
+  const int sh = E - e + 3;  // >= 4 for normal v; a subnormal group may need a left shift
+  const unsigned long long F = (M == 0 || sh >= 64) ? 0ull : (sh >= 0 ? (M >> sh) : (M << -sh));
+  neg = (unsigned)(bits >> 63);
+  return F;
+}
+
+template <typename Store>
+__device__ __forceinline__ void oz_digits(double v, int E, Store store) {
+  unsigned neg;
+  const unsigned long long F = oz_fixed(v, E, neg);
+#pragma unroll
+  for (int s = 0; s < kOzSlices; ++s) {
+    const int d = (int)((F >> (42 - 7 * s)) & 127ull);
+    store(s, __int2bfloat16_rn(neg ? -d : d));
+  }
+}
+
+// The digits of eight values, d[s] the eight of slice s: two values at a time,
+// 0x4300 | digit the bf16 128 + digit, and one packed multiply-add
+// +-(128 + digit) -+ 128 (a conversion a digit runs at a quarter of that rate).
+__device__ __forceinline__ void oz_digits8(const double (&v)[8], int E, uint4 (&d)[kOzSlices]) {
+  unsigned long long F[8];
+  unsigned neg[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) F[u] = oz_fixed(v[u], E, neg[u]);
+  unsigned w[kOzSlices][4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const unsigned sg = neg[2 * p] << 15 | neg[2 * p + 1] << 31, f = 0x3f803f80u | sg, a = 0xc300c300u ^ sg;
+#pragma unroll
+    for (int s = 0; s < kOzSlices; ++s) {
+      const unsigned t = (__byte_perm((unsigned)(F[2 * p] >> (42 - 7 * s)), (unsigned)(F[2 * p + 1] >> (42 - 7 * s)),
+                                      0x5410) & 0x007f007fu) | 0x43004300u;
+      const __nv_bfloat162 r = __hfma2(*reinterpret_cast<const __nv_bfloat162 *>(&t),
+                                       *reinterpret_cast<const __nv_bfloat162 *>(&f),
+                                       *reinterpret_cast<const __nv_bfloat162 *>(&a));
+      w[s][p] = *reinterpret_cast<const unsigned *>(&r);
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < kOzSlices; ++s) d[s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+}
+#endif
+
 // Leaf size and rank the tensor-core residual supports (else the double-word one runs).
 inline bool oz_supported(int m, int r) { return m % kOzChunk == 0 && m <= 256 && r >= 8 && r <= 64 && r % 8 == 0; }
 
