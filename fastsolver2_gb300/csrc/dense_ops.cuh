@@ -21,6 +21,19 @@ template <typename T> __device__ __forceinline__ void swap_vals(T &a, T &b) {
   b = t;
 }
 
+// 1 / x to FP64 accuracy for |x| in 2^-960 .. 2^960 (rcp_usual): the third-order
+// iteration y <- y (1 + e + e^2), e = 1 - x y, on the hardware's approximation,
+// which triples its correct bits (20); three FMAs where a division takes 440 clocks.
+__device__ __forceinline__ double newton_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ bool rcp_usual(double x) {
+  return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 63u < 1921u;
+}
+
 // In-place LU with partial pivoting of the m x m matrix A (lda).  piv gets the
 // 1-based LAPACK pivots.  *info = 0, or k+1 for the first zero pivot k.  The
 // pivot is the first row of maximal |a| (IDAMAX, netlib_blas/idamax.f:52).

@@ -58,16 +58,6 @@ struct LuOut {
 };
 }  // namespace
 
-// 1 / x to FP64 accuracy for a normal x of moderate size: Newton's iteration
-// y <- y + y (1 - x y) on the hardware's approximation, which doubles its
-// correct bits (20) twice.
-__device__ __forceinline__ double newton_rcp(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-
 // Rows [k0, k0 + 32) of block columns [k0, k0 + 32): see above.  A [block][m][m]
 // is worked on in place; W [block][32][m] (column c at + c m), R [block][m][32]
 // (column j at + 32 j), perm [block][m]: the original row at each position.
@@ -120,16 +110,12 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, int nc, cons
     mp = __reduce_min_sync(0xffffffffu, open && hi == mh && lo == ml ? (unsigned)pos : 0xffffu);
     return mp == 0xffffu ? lane == 0 : (open && (unsigned)pos == mp);
   };
-  auto usual = [](double v) {  // |v| in 2^-960 .. 2^960: its reciprocal is normal
-    const unsigned e = ((unsigned)__double2hiint(v) >> 20) & 0x7ffu;
-    return e - 63u < 1921u;
-  };
   // the candidate's row, reciprocal and key into buffer b
 #define HODLR_GJ_PUBLISH(c, b)                                                                    \
   if (real) {                                                                                     \
     if (cand) {                                                                                   \
       sBest[b][warp] = make_uint4(mh, ml, mp, tid);                                               \
-      sRcp[b][warp] = usual(a[c]) ? rc : ((__double2hiint(a[c]) & 0x7fffffff) | __double2loint(a[c])) ? 1.0 / a[c] : 0.0; \
+      sRcp[b][warp] = rcp_usual(a[c]) ? rc : ((__double2hiint(a[c]) & 0x7fffffff) | __double2loint(a[c])) ? 1.0 / a[c] : 0.0; \
       _Pragma("unroll") for (int j = c; j < kNb; ++j) sU[b][warp][j] = a[j];                      \
     }                                                                                             \
   }

@@ -510,7 +510,7 @@ static int leaf_solve(hodlr_ctx *h, T *X, long long ldx, int ncols, bool trans, 
           launch_leaf_apply<T>(Dinv, h->m, h->nleaf, X, ldx, ncols, trans, skip, h->st));
   else
     PHASE(h, HODLR_PHASE_LEAF_SOLVE,
-          launch_leaf_getrs<T>(LUptr<T>(h), h->ipiv, h->m, h->nleaf, X, ldx, ncols, trans, skip, h->st));
+          launch_leaf_getrs<T>(LUptr<T>(h), h->ipiv, h->m, h->nleaf, X, ldx, ncols, trans, skip, h->dst, h->st));
   return HODLR_OK;
 }
 

@@ -72,7 +72,8 @@ cudaError_t launch_leaf_inverse_blocked(const T *LU, const int *ipiv, int m, int
 // *skip != 0 the kernel returns immediately.
 template <typename T>
 cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T *X, long long ldx,
-                              int ncols, bool trans, const int *skip, cudaStream_t s);
+                              int ncols, bool trans, const int *skip, DevStatus *st,
+                              cudaStream_t s);
 
 // ----------------------------------------------------------- level steps
 // K3: Out_b = A_b^T X_b (r x C, FP64 result) for batches b in [0, nbatch),

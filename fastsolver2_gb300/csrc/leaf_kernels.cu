@@ -6,12 +6,15 @@
 // memory when it fits) and the solves against all right-hand-side columns
 // are one launch over (leaf, column tile).
 #include <algorithm>
+#include <cstdlib>
 
 #include "dense_ops.cuh"
 #include "kernels.cuh"
 #include "reg_factor.cuh"
 
 namespace hodlr {
+
+bool f64_update_tc_try(const UpdateArgs &a, DevStatus *st, cudaStream_t s, cudaError_t &err);
 
 template <typename T, bool SMEM>
 __global__ void __launch_bounds__(256)
@@ -118,6 +121,156 @@ leaf_getrs_kernel(const T *__restrict__ LU, const int *__restrict__ ipiv, int m,
   }
 }
 
+// Quotients by one divisor, by its reciprocal in two parts: rounded as the division
+// rounds but for extreme exponents, which are left to it.
+struct Quotient {
+  double u, hi, lo;
+  int ok;
+  __device__ __forceinline__ static Quotient by(double u) {
+    const double hi = 1.0 / u;
+    return Quotient{u, hi, fma(-u, hi, 1.0) * hi, fabs(u) > 1e-280 && fabs(u) < 1e280};
+  }
+  __device__ __forceinline__ double of(double x) const {  // x / u
+    const double q = fma(x, hi, x * lo);
+    return ok && isfinite(q) ? q : x / u;
+  }
+};
+
+// X := D^{-1} X in FP64 for many columns: 32-row diagonal blocks in launches of
+// their own -- 32 columns a CTA, lane = column, each of the four warps with every
+// fourth row in registers, row k passed through shared memory once it is done, a
+// step a barrier and up to eight FMAs --, the updates of the other rows on the
+// tensor cores (f64_update_tc.cu).  Bound by the FP64 pipe in the diagonal blocks
+// (2 x 496 FMAs a column and block) and by the updates, half each: 2048 leaves of
+// 100 rows, 143 columns and then 5: 5.0 ms, 22.1 with one CTA a leaf and column
+// tile doing it all by FMAs; 512 leaves of 300 rows, 122 columns 4.1 ms, 22.2.
+__global__ void __launch_bounds__(256) leaf_interchange_kernel(const int *__restrict__ ipiv, int m, double *X,
+                                                               long long ldx, int ncols, int ct, const int *skip) {
+  if (skip && *skip) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double *sX = reinterpret_cast<double *>(smem_raw);  // [ct][m]
+  int *sfrom = reinterpret_cast<int *>(sX + (size_t)m * ct), *spiv = sfrom + m;
+  const int leaf = blockIdx.y, c0 = blockIdx.x * ct, nc = min(ct, ncols - c0), tid = threadIdx.x;
+  double *Xg = X + (long long)leaf * m + (long long)c0 * ldx;
+  for (int i = tid; i < m; i += 256) spiv[i] = ipiv[(long long)leaf * m + i] - 1;
+  __syncthreads();
+  for (int i = tid; i < m; i += 256) {
+    int from = i;  // row i of P X
+    for (int k = m - 1; k >= 0; --k) {
+      const int p = spiv[k];
+      from = from == k ? p : from == p ? k : from;
+    }
+    sfrom[i] = from;
+  }
+  for (int c = tid >> 5; c < nc; c += 8)
+    for (int i = tid & 31; i < m; i += 32) sX[c * m + i] = Xg[i + (long long)c * ldx];
+  __syncthreads();
+  for (int c = tid >> 5; c < nc; c += 8)
+    for (int i = tid & 31; i < m; i += 32)
+      if (sfrom[i] != i) Xg[i + (long long)c * ldx] = sX[c * m + sfrom[i]];
+}
+
+template <bool UPPER>
+__global__ void __launch_bounds__(128) leaf_diag_kernel(const double *__restrict__ LU, int m, int k0, double *X,
+                                                        long long ldx, int ncols, const int *skip) {
+  if (skip && *skip) return;
+  __shared__ double sA[32][32], sX[32][33], sK[2][32];  // sA[column][row], sX[column][row]
+  __shared__ Quotient sR[32];
+  const int leaf = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kb = min(32, m - k0);
+  const int c0 = blockIdx.x * 32;
+  const double *A = LU + (long long)leaf * m * m + k0 + (long long)k0 * m;
+  double *Xg = X + (long long)leaf * m + k0 + (long long)c0 * ldx;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int c = warp + 4 * i;
+    sA[c][lane] = lane < kb && c < kb ? A[lane + (long long)c * m] : c == lane ? 1.0 : 0.0;
+    sX[c][lane] = lane < kb && c0 + c < ncols ? Xg[lane + (long long)c * ldx] : 0.0;
+  }
+  __syncthreads();
+  if (UPPER) {
+    if (tid < 32) sR[tid] = Quotient::by(sA[tid][tid]);
+    __syncthreads();
+  }
+  double x[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) x[q] = sX[lane][4 * q + warp];
+#pragma unroll
+  for (int step = 0; step < 32; ++step) {
+    const int k = UPPER ? 31 - step : step;
+    if (warp == (k & 3)) {
+      if (UPPER) x[k / 4] = sR[k].of(x[k / 4]);
+      sK[k & 1][lane] = x[k / 4];
+    }
+    __syncthreads();
+    const double xk = sK[k & 1][lane];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (UPPER ? 4 * q > k : 4 * q + 3 < k) continue;
+      if (UPPER ? 4 * q + warp < k : 4 * q + warp > k) x[q] -= sA[k][4 * q + warp] * xk;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) sX[lane][4 * q + warp] = x[q];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int c = warp + 4 * i;
+    if (lane < kb && c0 + c < ncols) Xg[lane + (long long)c * ldx] = sX[c][lane];
+  }
+}
+
+// The line: 4 m / 32 launches of some 10 us each against the one of
+// leaf_getrs_kernel, whose time grows with the elements: 16 leaves of 180 rows, 20
+// columns 0.19 ms there and 0.25 here; 32 leaves of 100 rows, 32 columns 0.16 and
+// 0.16; 32 of 180 rows, 70 columns 0.77 and 0.44; 64 of 50 rows, 50 columns 0.19
+// and 0.12.  Up to 8 columns would fill a quarter of a tile: 2048 leaves of 100
+// rows, 5 columns 0.91 and 1.10.
+static bool leaf_getrs_on_tensor_cores(int m, int nleaf, int ncols) {
+  const char *no_tc = getenv("HODLR_NO_TCGEN05");
+  return !(no_tc && no_tc[0] == '1') && m > 32 && ncols > 8 && (long long)nleaf * ncols * m >= 1 << 17;
+}
+
+static cudaError_t leaf_getrs_blocked(const double *LU, const int *ipiv, int m, int nleaf, double *X, long long ldx,
+                                      int ncols, const int *skip, DevStatus *st, cudaStream_t s) {
+  const int ct = std::max(1, std::min(8, (int)(96 * 1024 / ((size_t)m * sizeof(double)))));
+  const size_t bytes = (size_t)m * (ct * sizeof(double) + 2 * sizeof(int));
+  cudaError_t e = allow_dyn_smem(leaf_interchange_kernel, bytes);
+  if (e != cudaSuccess) return e;
+  HODLR_LAUNCH(leaf_interchange_kernel, dim3(ceil_div(ncols, ct), nleaf), 256, bytes, s, ipiv, m, X, ldx, ncols, ct,
+               skip);
+  const dim3 grid(ceil_div(ncols, 32), nleaf);
+  auto update = [&](int k0, int r0, int r1) {  // rows [r0, r1) -= A(rows, block) X(block)
+    UpdateArgs ua{};
+    ua.A = LU + r0 + (long long)k0 * m;
+    ua.lda = m;
+    ua.a_bstride = (long long)m * m;
+    ua.B = X + k0;
+    ua.ldb = ldx;
+    ua.b_s1 = 2LL * m;
+    ua.b_s2 = m;
+    ua.C = X + r0;
+    ua.ldc = ldx;
+    ua.c_bstride = m;
+    ua.M = r1 - r0;
+    ua.N = ncols;
+    ua.K = std::min(32, m - k0);
+    ua.nbatch = nleaf;
+    ua.alpha = -1.0;
+    ua.skip = skip;
+    return f64_update_tc_try(ua, st, s, e) ? e : cudaErrorInvalidValue;
+  };
+  const int last = (m - 1) / 32 * 32;
+  for (int k0 = 0; k0 <= last; k0 += 32) {
+    HODLR_LAUNCH(leaf_diag_kernel<false>, grid, 128, 0, s, LU, m, k0, X, ldx, ncols, skip);
+    if (k0 < last && (e = update(k0, k0 + 32, m)) != cudaSuccess) return e;
+  }
+  for (int k0 = last; k0 >= 0; k0 -= 32) {
+    HODLR_LAUNCH(leaf_diag_kernel<true>, grid, 128, 0, s, LU, m, k0, X, ldx, ncols, skip);
+    if (k0 > 0 && (e = update(k0, 0, k0)) != cudaSuccess) return e;
+  }
+  return cudaGetLastError();
+}
+
 static constexpr size_t kSmemCap = 220 * 1024;
 
 template <typename K>
@@ -149,7 +302,13 @@ cudaError_t launch_leaf_getrf(const double *D, long long d_ld, long long d_strid
   if (m == 64) return launch_reg<T, 64>(D, d_ld, d_stride, LU, ipiv, nleaf, st, Dinv, s);
   if (m == 128) return launch_reg<T, 128>(D, d_ld, d_stride, LU, ipiv, nleaf, st, Dinv, s);
   const size_t bytes = (size_t)m * (m + 1) * sizeof(T) + (size_t)m * 4;
-  if (bytes <= kSmemCap) {
+  // In FP64 the panels of leaf_blocked.cu from 96 rows on, where the one CTA of
+  // leaf_getrf_kernel spends a leaf's time on barriers and FMAs: 2048 leaves of 100
+  // rows 1.88 ms by panels and 3.06 here, 1024 of 150 rows 1.76 and 5.46, 4 of 100
+  // rows 0.25 and 0.35; 256 of 72 rows 0.29 and 0.25.
+  const char *no_tc = getenv("HODLR_NO_TCGEN05");
+  const bool panels = sizeof(T) == 8 && m >= 96 && !Dinv && !(no_tc && no_tc[0] == '1');
+  if (bytes <= kSmemCap && !panels) {
     auto k = leaf_getrf_kernel<T, true>;
     cudaError_t e = set_smem(k, bytes);
     if (e != cudaSuccess) return e;
@@ -163,8 +322,11 @@ cudaError_t launch_leaf_getrf(const double *D, long long d_ld, long long d_strid
 
 template <typename T>
 cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T *X, long long ldx,
-                              int ncols, bool trans, const int *skip, cudaStream_t s) {
+                              int ncols, bool trans, const int *skip, DevStatus *st, cudaStream_t s) {
   if (ncols <= 0 || nleaf <= 0) return cudaSuccess;
+  if constexpr (sizeof(T) == 8)
+    if (!trans && leaf_getrs_on_tensor_cores(m, nleaf, ncols))
+      return leaf_getrs_blocked(LU, ipiv, m, nleaf, X, ldx, ncols, skip, st, s);
   const size_t lu_bytes = (size_t)m * m * sizeof(T);
   const size_t piv_bytes = (size_t)m * sizeof(int) + 16;
   // FP32: keep two CTAs per SM; FP64 is DFMA-bound, one CTA per SM suffices.
@@ -201,8 +363,8 @@ template cudaError_t launch_leaf_getrf<double>(const double *, long long, long l
 template cudaError_t launch_leaf_getrf<float>(const double *, long long, long long, float *, int *, int,
                                               int, DevStatus *, float *, cudaStream_t);
 template cudaError_t launch_leaf_getrs<double>(const double *, const int *, int, int, double *, long long,
-                                               int, bool, const int *, cudaStream_t);
+                                               int, bool, const int *, DevStatus *, cudaStream_t);
 template cudaError_t launch_leaf_getrs<float>(const float *, const int *, int, int, float *, long long, int,
-                                              bool, const int *, cudaStream_t);
+                                              bool, const int *, DevStatus *, cudaStream_t);
 
 }  // namespace hodlr
