@@ -1642,7 +1642,8 @@ int hodlr_set_lowrank(hodlr_handle h, int level, const double *U, int64_t ldu, c
   });
 }
 
-int hodlr_factor(hodlr_handle h) {
+// hodlr_factor in two parts: its work enqueued, its outcome awaited.
+static int factor_begin(hodlr_handle h) {
   if (!h) return set_err(HODLR_ERR_INVALID_ARG, "null handle");
   TuningScope tscope(&h->tune);
   if (!h->has_D) return set_err(HODLR_ERR_NOT_FACTORED, "leaf blocks not set");
@@ -1686,6 +1687,10 @@ int hodlr_factor(hodlr_handle h) {
   CKS(rc);
   if (sv) std::fill(h->vsrc.begin(), h->vsrc.end(), nullptr);
   CK(cudaEventRecord(h->ev[1], h->st));
+  return HODLR_OK;
+}
+
+static int factor_end(hodlr_handle h) {
   int fst = sync_status(h, nullptr);
   collect_phases(h);
   CKS(fst);
@@ -1694,6 +1699,42 @@ int hodlr_factor(hodlr_handle h) {
   h->lu_stale = leaf_inverse_only(h);
   return HODLR_OK;
 }
+
+int hodlr_factor(hodlr_handle h) {
+  CKS(factor_begin(h));
+  return factor_end(h);
+}
+
+// Independent handles of one stream factored side by side, handle i's work on
+// streams[i] between two points of `s`.  The first failure is returned, *bad its
+// index; handles after one whose work could not be enqueued are left as they are.
+namespace hodlr {
+int hodlr_factor_many(hodlr_handle *h, int count, cudaStream_t s, const cudaStream_t *streams, cudaEvent_t fork, int *bad) {
+  CK(cudaEventRecord(fork, s));
+  int begun = 0, rc = HODLR_OK;
+  for (; begun < count && rc == HODLR_OK; ++begun) {
+    CK(cudaStreamWaitEvent(streams[begun], fork, 0));
+    h[begun]->st = streams[begun];
+    rc = factor_begin(h[begun]);
+  }
+  int first = rc == HODLR_OK ? count : begun - 1;
+  std::string why = rc == HODLR_OK ? "" : hodlr_last_error_string();
+  for (int i = begun - 1; i >= 0; --i) {
+    if (!(rc != HODLR_OK && i == begun - 1)) {
+      const int e = factor_end(h[i]);
+      if (e != HODLR_OK) {
+        first = i;
+        rc = e;
+        why = hodlr_last_error_string();
+      }
+    }
+    cudaStreamSynchronize(streams[i]);
+    h[i]->st = s;
+  }
+  *bad = first;
+  return rc == HODLR_OK ? rc : set_err(rc, why);
+}
+}  // namespace hodlr
 
 static int solve_impl(hodlr_handle h, double *B, int64_t ldb, int nrhs, hodlr_solve_info *info, bool trans) {
   if (!h || !B) return set_err(HODLR_ERR_INVALID_ARG, "null argument");
