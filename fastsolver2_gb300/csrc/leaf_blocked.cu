@@ -407,7 +407,6 @@ __global__ void __launch_bounds__(256) leaf_inverse_blocked_kernel(const T *__re
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *sX = reinterpret_cast<T *>(smem_raw);                 // m x 32, ld m
   T *sP = sX + (size_t)m * kTrailCols;                      // panel pass: 128 x 32, [k * 128 + r]
-  T *sD = sP + kTrailRows * kPanelNb;                       // diagonal block 32 x 32, ld 32
   const int leaf = blockIdx.y, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, grp = tid >> 5;
   const T *A = LU + (long long)leaf * m * m;
   const int *piv = ipiv + (long long)leaf * m;
@@ -461,40 +460,61 @@ __global__ void __launch_bounds__(256) leaf_inverse_blocked_kernel(const T *__re
         }
     }
   };
+  // a diagonal block: a warp takes four of the 32 columns, lane = row, the block's
+  // rows of the factors in registers
+  T d[kPanelNb];
   auto load_diag = [&](int kb0, int kbn) {
+#pragma unroll
+    for (int k = 0; k < kPanelNb; ++k)
+      d[k] = lane < kbn && k < kbn ? A[(kb0 + lane) + (long long)(kb0 + k) * m] : T(k == lane);
+  };
+  constexpr int CW = kTrailCols / 8;
+  T x[CW];
+  auto load_x = [&](int kb0, int kbn) {
     __syncthreads();
-    for (int e = tid; e < kbn * kbn; e += nt) {
-      const int i = e % kbn, k = e / kbn;
-      sD[i + k * kPanelNb] = A[(kb0 + i) + (long long)(kb0 + k) * m];
-    }
-    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < CW; ++c) x[c] = lane < kbn ? sX[kb0 + lane + (CW * grp + c) * m] : T(0);
+  };
+  auto store_x = [&](int kb0, int kbn) {
+#pragma unroll
+    for (int c = 0; c < CW; ++c)
+      if (lane < kbn) sX[kb0 + lane + (CW * grp + c) * m] = x[c];
   };
   // L Y = P X, unit lower, 32-row blocks top down
   for (int kb0 = 0; kb0 < m; kb0 += kPanelNb) {
     const int kbn = min(kPanelNb, m - kb0);
     load_diag(kb0, kbn);
-    for (int k = 0; k + 1 < kbn; ++k) {
-      for (int e = tid; e < (kbn - k - 1) * kTrailCols; e += nt) {
-        const int i = k + 1 + e % (kbn - k - 1), c = e / (kbn - k - 1);
-        sX[(kb0 + i) + c * m] -= sX[(kb0 + k) + c * m] * sD[i + k * kPanelNb];
+    load_x(kb0, kbn);
+#pragma unroll
+    for (int k = 0; k + 1 < kPanelNb; ++k)
+#pragma unroll
+      for (int c = 0; c < CW; ++c) {
+        const T xk = __shfl_sync(0xffffffffu, x[c], k);
+        if (lane > k) x[c] -= xk * d[k];
       }
-      __syncthreads();
-    }
+    store_x(kb0, kbn);
     if (kb0 + kbn < m) panel_update(kb0, kbn, kb0 + kbn, m);
   }
   // U X = Y, 32-row blocks bottom up
   for (int kb0 = ((m - 1) / kPanelNb) * kPanelNb; kb0 >= 0; kb0 -= kPanelNb) {
     const int kbn = min(kPanelNb, m - kb0);
     load_diag(kb0, kbn);
-    for (int k = kbn - 1; k >= 0; --k) {
-      if (tid < kTrailCols) sX[(kb0 + k) + tid * m] /= sD[k + k * kPanelNb];
-      __syncthreads();
-      for (int e = tid; e < k * kTrailCols; e += nt) {
-        const int i = e % k, c = e / k;
-        sX[(kb0 + i) + c * m] -= sX[(kb0 + k) + c * m] * sD[i + k * kPanelNb];
+    T u = T(1);  // the lane's pivot
+#pragma unroll
+    for (int k = 0; k < kPanelNb; ++k)
+      if (k == lane) u = d[k];
+    load_x(kb0, kbn);
+#pragma unroll
+    for (int k = kPanelNb - 1; k >= 0; --k) {
+      if (k >= kbn) continue;
+#pragma unroll
+      for (int c = 0; c < CW; ++c) {
+        if (lane == k) x[c] /= u;
+        const T xk = __shfl_sync(0xffffffffu, x[c], k);
+        if (lane < k) x[c] -= xk * d[k];
       }
-      __syncthreads();
     }
+    store_x(kb0, kbn);
     if (kb0 > 0) panel_update(kb0, kbn, 0, kb0);
   }
   __syncthreads();
@@ -505,7 +525,7 @@ __global__ void __launch_bounds__(256) leaf_inverse_blocked_kernel(const T *__re
 }
 
 size_t leaf_inverse_blocked_smem(int m, int elem_bytes) {
-  return (size_t)elem_bytes * ((size_t)m * kTrailCols + (size_t)kTrailRows * kPanelNb + (size_t)kPanelNb * kPanelNb);
+  return (size_t)elem_bytes * ((size_t)m * kTrailCols + (size_t)kTrailRows * kPanelNb);
 }
 
 template <typename T>
