@@ -394,138 +394,145 @@ __global__ void __launch_bounds__(256) leaf_trail_kernel(T *LU, int m, int j0, i
 
 // Explicit inverses D^{-1} = U^{-1} L^{-1} P from the LU factors of every leaf:
 // CTA (tile, leaf) owns columns [c0, c0 + 32) of the inverse, all m rows in
-// shared memory.  The identity's columns get the interchanges, then a blocked
-// unit-lower solve (32-row diagonal blocks in DTRSM's order, the rows below
-// updated by the block's L panel in passes of 128 rows) and a blocked upper
-// solve from the bottom (diagonal blocks by division, the rows above updated
-// by the block's U panel) -- the DGETRS order on the identity.  (For solves
-// with a few right-hand sides the one-CTA-per-column-tile kernel of
-// launch_leaf_getrs, which spreads the columns over every SM, is faster.)
+// shared memory, a row's 32 columns side by side.  The identity's columns get
+// the interchanges, then a blocked unit-lower solve (32-row diagonal blocks, the
+// rows below updated by the block's L panel in passes of 256 rows) and a blocked
+// upper solve from the bottom (diagonal blocks by division, the rows above
+// updated by the block's U panel) -- the DGETRS order on the identity.  (For
+// solves with a few right-hand sides launch_leaf_getrs, which spreads the columns
+// over every SM, is faster.)
+//
+// A diagonal block takes no barrier: a warp has four of the columns, lane = row, a
+// step a shuffle and an FMA a column.  In a pass a thread has 4 rows x 8 columns:
+// 6 shared-memory wavefronts a warp for 32 FMAs.  1024 FP32 leaves of 256 rows take
+// 3.7 ms, 4.1 with 4 x 4 a thread.
+constexpr int kInvRows = 256;  // rows of a pass
 template <typename T>
 __global__ void __launch_bounds__(256) leaf_inverse_blocked_kernel(const T *__restrict__ LU,
                                                                    const int *__restrict__ ipiv, int m, T *Dinv) {
+  constexpr int NB = kPanelNb, LD = kTrailCols + 4;
+  struct alignas(16) Four {
+    T v[4];
+  };
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sX = reinterpret_cast<T *>(smem_raw);                 // m x 32, ld m
-  T *sP = sX + (size_t)m * kTrailCols;                      // panel pass: 128 x 32, [k * 128 + r]
-  const int leaf = blockIdx.y, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, grp = tid >> 5;
+  T *sX = reinterpret_cast<T *>(smem_raw);  // m x 32, column c of row i at [i * LD + c]
+  T *sP = sX + (size_t)m * LD;              // panel pass: 256 x 32, [k * 256 + r]
+  int *spiv = reinterpret_cast<int *>(sP);  // (before the first pass)
+  const int leaf = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const T *A = LU + (long long)leaf * m * m;
-  const int *piv = ipiv + (long long)leaf * m;
   const int c0 = blockIdx.x * kTrailCols, nc = min(kTrailCols, m - c0);
   T *out = Dinv + (long long)leaf * m * m + (long long)c0 * m;
-  for (int e = tid; e < m * kTrailCols; e += nt) {
-    const int i = e % m, c = e / m;
-    sX[e] = (c < nc && i == c0 + c) ? T(1) : T(0);
-  }
+  for (int i = tid; i < m; i += 256) spiv[i] = ipiv[(long long)leaf * m + i] - 1;
   __syncthreads();
-  if (tid < nc)
-    for (int k = 0; k < m; ++k) {
-      const int p = piv[k] - 1;
-      if (p != k) swap_vals(sX[k + tid * m], sX[p + tid * m]);
+  for (int i = tid; i < m; i += 256) {
+    int from = i;  // row i of P I
+    for (int k = m - 1; k >= 0; --k) {
+      const int p = spiv[k];
+      from = from == k ? p : from == p ? k : from;
     }
-  // rows [r0, r0 + nr) -= A(rows, kb block) * X(kb block rows, :), the panel streamed in 128-row passes
+    for (int c = 0; c < kTrailCols; ++c) sX[i * LD + c] = from == c0 + c ? T(1) : T(0);
+  }
+  // rows [r0, r1) -= A(rows, kb block) X(kb block rows, :)
   auto panel_update = [&](int kb0, int kbn, int r0, int r1) {
-    for (int p0 = r0; p0 < r1; p0 += kTrailRows) {
-      const int nr = min(kTrailRows, r1 - p0);
+    const int g = warp & 3, h = warp >> 2;  // columns 8 g + (0..7), rows 128 h + lane + 32 (0..3) of a pass
+    for (int p0 = r0; p0 < r1; p0 += kInvRows) {
+      const int nr = min(kInvRows, r1 - p0);
       __syncthreads();
-      for (int e = tid; e < kTrailRows * kbn; e += nt) {
-        const int r = e % kTrailRows, k = e / kTrailRows;
-        sP[k * kTrailRows + r] = r < nr ? A[(p0 + r) + (long long)(kb0 + k) * m] : T(0);
-      }
+#pragma unroll
+      for (int k = 0; k < NB; ++k)
+        sP[k * kInvRows + tid] = tid < nr && k < kbn ? A[(p0 + tid) + (long long)(kb0 + k) * m] : T(0);
       __syncthreads();
-      T acc[4][4];
+      if (128 * h >= nr) continue;
+      T acc[4][8];
+      T *Xr = sX + (p0 + 128 * h + lane) * LD + 8 * g;
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int r = lane + 32 * a;
-          acc[a][b] = r < nr ? sX[(p0 + r) + (4 * grp + b) * m] : T(0);
+        for (int q = 0; q < 2; ++q) {
+          Four f{};
+          if (128 * h + lane + 32 * a < nr) f = *reinterpret_cast<const Four *>(Xr + 32 * a * LD + 4 * q);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[a][4 * q + e] = f.v[e];
         }
       for (int k = 0; k < kbn; ++k) {
-        T l[4], u[4];
+        T l[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) l[a] = sP[k * kTrailRows + lane + 32 * a];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) u[b] = sX[(kb0 + k) + (4 * grp + b) * m];
+        for (int a = 0; a < 4; ++a) l[a] = sP[k * kInvRows + 128 * h + lane + 32 * a];
+        const Four u0 = *reinterpret_cast<const Four *>(sX + (kb0 + k) * LD + 8 * g);
+        const Four u1 = *reinterpret_cast<const Four *>(sX + (kb0 + k) * LD + 8 * g + 4);
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] -= l[a] * u[b];
+          for (int e = 0; e < 4; ++e) {
+            acc[a][e] -= l[a] * u0.v[e];
+            acc[a][4 + e] -= l[a] * u1.v[e];
+          }
       }
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int r = lane + 32 * a;
-          if (r < nr) sX[(p0 + r) + (4 * grp + b) * m] = acc[a][b];
+        for (int q = 0; q < 2; ++q) {
+          Four f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) f.v[e] = acc[a][4 * q + e];
+          if (128 * h + lane + 32 * a < nr) *reinterpret_cast<Four *>(Xr + 32 * a * LD + 4 * q) = f;
         }
     }
   };
-  // a diagonal block: a warp takes four of the 32 columns, lane = row, the block's
-  // rows of the factors in registers
-  T d[kPanelNb];
-  auto load_diag = [&](int kb0, int kbn) {
+  // a diagonal block: the block's rows of the factors in registers
+  T d[NB];
+  Four x;
+  auto load = [&](int kb0, int kbn) {
 #pragma unroll
-    for (int k = 0; k < kPanelNb; ++k)
+    for (int k = 0; k < NB; ++k)
       d[k] = lane < kbn && k < kbn ? A[(kb0 + lane) + (long long)(kb0 + k) * m] : T(k == lane);
-  };
-  constexpr int CW = kTrailCols / 8;
-  T x[CW];
-  auto load_x = [&](int kb0, int kbn) {
     __syncthreads();
-#pragma unroll
-    for (int c = 0; c < CW; ++c) x[c] = lane < kbn ? sX[kb0 + lane + (CW * grp + c) * m] : T(0);
+    x = Four{};
+    if (lane < kbn) x = *reinterpret_cast<const Four *>(sX + (kb0 + lane) * LD + 4 * warp);
   };
-  auto store_x = [&](int kb0, int kbn) {
-#pragma unroll
-    for (int c = 0; c < CW; ++c)
-      if (lane < kbn) sX[kb0 + lane + (CW * grp + c) * m] = x[c];
+  auto store = [&](int kb0, int kbn) {
+    if (lane < kbn) *reinterpret_cast<Four *>(sX + (kb0 + lane) * LD + 4 * warp) = x;
   };
-  // L Y = P X, unit lower, 32-row blocks top down
-  for (int kb0 = 0; kb0 < m; kb0 += kPanelNb) {
-    const int kbn = min(kPanelNb, m - kb0);
-    load_diag(kb0, kbn);
-    load_x(kb0, kbn);
+  for (int kb0 = 0; kb0 < m; kb0 += NB) {  // L Y = P X
+    const int kbn = min(NB, m - kb0);
+    load(kb0, kbn);
 #pragma unroll
-    for (int k = 0; k + 1 < kPanelNb; ++k)
+    for (int k = 0; k + 1 < NB; ++k)
 #pragma unroll
-      for (int c = 0; c < CW; ++c) {
-        const T xk = __shfl_sync(0xffffffffu, x[c], k);
-        if (lane > k) x[c] -= xk * d[k];
+      for (int c = 0; c < 4; ++c) {
+        const T xk = __shfl_sync(0xffffffffu, x.v[c], k);
+        if (lane > k) x.v[c] -= xk * d[k];
       }
-    store_x(kb0, kbn);
+    store(kb0, kbn);
     if (kb0 + kbn < m) panel_update(kb0, kbn, kb0 + kbn, m);
   }
-  // U X = Y, 32-row blocks bottom up
-  for (int kb0 = ((m - 1) / kPanelNb) * kPanelNb; kb0 >= 0; kb0 -= kPanelNb) {
-    const int kbn = min(kPanelNb, m - kb0);
-    load_diag(kb0, kbn);
+  for (int kb0 = (m - 1) / NB * NB; kb0 >= 0; kb0 -= NB) {  // U X = Y
+    const int kbn = min(NB, m - kb0);
+    load(kb0, kbn);
     T u = T(1);  // the lane's pivot
 #pragma unroll
-    for (int k = 0; k < kPanelNb; ++k)
+    for (int k = 0; k < NB; ++k)
       if (k == lane) u = d[k];
-    load_x(kb0, kbn);
 #pragma unroll
-    for (int k = kPanelNb - 1; k >= 0; --k) {
+    for (int k = NB - 1; k >= 0; --k) {
       if (k >= kbn) continue;
 #pragma unroll
-      for (int c = 0; c < CW; ++c) {
-        if (lane == k) x[c] /= u;
-        const T xk = __shfl_sync(0xffffffffu, x[c], k);
-        if (lane < k) x[c] -= xk * d[k];
+      for (int c = 0; c < 4; ++c) {
+        if (lane == k) x.v[c] /= u;
+        const T xk = __shfl_sync(0xffffffffu, x.v[c], k);
+        if (lane < k) x.v[c] -= xk * d[k];
       }
     }
-    store_x(kb0, kbn);
+    store(kb0, kbn);
     if (kb0 > 0) panel_update(kb0, kbn, 0, kb0);
   }
   __syncthreads();
-  for (int e = tid; e < m * nc; e += nt) {
-    const int i = e % m, c = e / m;
-    out[i + (long long)c * m] = sX[i + c * m];
-  }
+  for (int c = warp; c < nc; c += 8)
+    for (int i = lane; i < m; i += 32) out[i + (long long)c * m] = sX[i * LD + c];
 }
 
 size_t leaf_inverse_blocked_smem(int m, int elem_bytes) {
-  return (size_t)elem_bytes * ((size_t)m * kTrailCols + (size_t)kTrailRows * kPanelNb);
+  return (size_t)elem_bytes * ((size_t)m * (kTrailCols + 4) + (size_t)kInvRows * kPanelNb);
 }
 
 template <typename T>
