@@ -173,7 +173,9 @@ struct hodlr_ctx {
   __nv_bfloat16 *Dsl = nullptr, *Usl = nullptr, *Vsl = nullptr, *Xsl = nullptr, *Tsl = nullptr;
   int *Dexp = nullptr, *Uexp = nullptr, *Vexp = nullptr, *Xexp = nullptr, *Texp = nullptr;
   size_t tbuf_elems = 0, eta_elems = 0, red_elems = 0;
-  DevStatus *dst = nullptr, *hst = nullptr;
+  DevStatus *dst = nullptr, *hst = nullptr;  // hst: pinned, or `status` of a handle for one call
+  DevStatus status{};
+  char *staging = nullptr;  // of a handle for one call: device memory for its host buffers
   // timing
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
   // set-time preparation on a side stream (hodlr_set_leaf_blocks /
@@ -224,11 +226,28 @@ struct hodlr_ctx {
   double phase_ms[HODLR_NUM_PHASES] = {};
   long long phase_n[HODLR_NUM_PHASES] = {};
 
+  // One device block holds every array of a small handle: first the sizes are
+  // added up (counting), then the arrays laid into it; any other request is an
+  // allocation of its own.
+  bool counting = false;
+  size_t block_bytes = 0, block_used = 0;
+  char *block = nullptr;
   template <typename T> T *alloc(size_t count, cudaError_t &err) {
-    void *p = nullptr;
     if (count == 0) count = 1;
-    err = cudaMalloc(&p, count * sizeof(T));
-    if (err == cudaSuccess) allocs.push_back(p);
+    const size_t bytes = (count * sizeof(T) + 255) / 256 * 256;
+    err = cudaSuccess;
+    if (counting) {
+      block_bytes += bytes;
+      return reinterpret_cast<T *>(256);  // no null, never used
+    }
+    void *p = nullptr;
+    if (block && block_used + bytes <= block_bytes) {
+      p = block + block_used;
+      block_used += bytes;
+    } else {
+      err = cudaMalloc(&p, count * sizeof(T));
+      if (err == cudaSuccess) allocs.push_back(p);
+    }
     return static_cast<T *>(p);
   }
   double *Ulev(int l) const { return U + (long long)l * n * r; }
@@ -346,7 +365,7 @@ static void free_ctx(hodlr_ctx *h) {
   clear_graphs(h);
   destroy_recs(h->eager_recs);
   for (void *p : h->allocs) cudaFree(p);
-  if (h->hst) cudaFreeHost(h->hst);
+  if (h->hst && h->hst != &h->status) cudaFreeHost(h->hst);
   for (auto &e : h->ev)
     if (e) cudaEventDestroy(e);
   if (h->pst) cudaStreamSynchronize(h->pst);
@@ -1245,46 +1264,15 @@ static int check_common(const hodlr_desc &d) {
   return HODLR_OK;
 }
 
-// Allocate a handle for one tree (sys_levels = {L}) or for a forest of
-// trees with the same leaf size and rank (sys_levels sorted in decreasing
-// order; d.n = sum of leaf * 2^L_i and d.levels = the largest L_i).
-static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, hodlr_ctx **out) {
-  hodlr_ctx *h = new hodlr_ctx();
-  h->d = d;
-  h->n = d.n;
-  h->m = d.leaf;
-  h->L = d.levels;
-  h->r = d.levels > 0 ? d.rank : std::max(1, d.rank);
-  h->nleaf = (int)(d.n / d.leaf);
-  h->kmax = d.nrhs_max;
-  h->mixed = d.precision == HODLR_PREC_MIXED;
-  h->has_level.assign(h->L, 0);
-  h->vsrc.assign(h->L, nullptr);
-  h->vsrc_ld.assign(h->L, 0);
-  h->nsys = (int)sys_levels.size();
-  h->forest = h->nsys > 1;
-  set_geometry(h, sys_levels);
-  if (d.stream) {
-    h->st = (cudaStream_t)d.stream;
-  } else {
-    cudaError_t e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
-    if (e != cudaSuccess) {
-      delete h;
-      return set_err(HODLR_ERR_CUDA, cudaGetErrorString(e));
-    }
-    h->own_stream = true;
-  }
-  plan_sizes(h);
+// The handle's device arrays.
+static int alloc_arrays(hodlr_ctx *h, const hodlr_desc &d) {
   const long long n = h->n;
   const int m = h->m, L = h->L, r = h->r, k = h->kmax;
   cudaError_t e = cudaSuccess;
 #define ALLOC(ptr, T, cnt)                                                    \
   do {                                                                        \
     ptr = h->alloc<T>((size_t)(cnt), e);                                      \
-    if (e != cudaSuccess) {                                                   \
-      free_ctx(h);                                                            \
-      return set_err(HODLR_ERR_OUT_OF_MEMORY, std::string("cudaMalloc ") + #ptr); \
-    }                                                                         \
+    if (e != cudaSuccess) return set_err(HODLR_ERR_OUT_OF_MEMORY, std::string("cudaMalloc ") + #ptr); \
   } while (0)
   ALLOC(h->D, double, (size_t)h->nleaf * m * m);
   ALLOC(h->U, double, (size_t)n * L * r);
@@ -1392,7 +1380,79 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
     }
     (void)cudaGetLastError();
   }
-  if (cudaMallocHost(&h->hst, sizeof(DevStatus)) != cudaSuccess) {
+  return HODLR_OK;
+}
+
+// A handle of up to this many bytes takes one allocation: at 2 MB and more a
+// cudaMalloc takes some 50 us and its cudaFree 40, each of the others 1 to 3.
+constexpr size_t kBlockMost = 64u << 20;
+
+// Allocate a handle for one tree (sys_levels = {L}) or for a forest of
+// trees with the same leaf size and rank (sys_levels sorted in decreasing
+// order; d.n = sum of leaf * 2^L_i and d.levels = the largest L_i).
+// one_call: the handle lives for one call, with `staging` bytes of device memory; its
+// status comes back to pageable memory (pinning a page and giving it back takes
+// 0.3 ms, each read 5 us more).
+static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, hodlr_ctx **out, bool one_call = false,
+                      size_t staging = 0) {
+  hodlr_ctx *h = new hodlr_ctx();
+  h->d = d;
+  h->n = d.n;
+  h->m = d.leaf;
+  h->L = d.levels;
+  h->r = d.levels > 0 ? d.rank : std::max(1, d.rank);
+  h->nleaf = (int)(d.n / d.leaf);
+  h->kmax = d.nrhs_max;
+  h->mixed = d.precision == HODLR_PREC_MIXED;
+  h->has_level.assign(h->L, 0);
+  h->vsrc.assign(h->L, nullptr);
+  h->vsrc_ld.assign(h->L, 0);
+  h->nsys = (int)sys_levels.size();
+  h->forest = h->nsys > 1;
+  set_geometry(h, sys_levels);
+  if (d.stream) {
+    h->st = (cudaStream_t)d.stream;
+  } else {
+    cudaError_t e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
+    if (e != cudaSuccess) {
+      delete h;
+      return set_err(HODLR_ERR_CUDA, cudaGetErrorString(e));
+    }
+    h->own_stream = true;
+  }
+  plan_sizes(h);
+  const long long n = h->n;
+  const int L = h->L, r = h->r;
+  cudaError_t e = cudaSuccess;
+  h->counting = true;
+  int rc = alloc_arrays(h, d);
+  if (staging) (void)h->alloc<char>(staging, e);
+  h->counting = false;
+  if (rc == HODLR_OK && h->block_bytes <= kBlockMost) {
+    void *p = nullptr;
+    if (cudaMalloc(&p, h->block_bytes) == cudaSuccess) {
+      h->block = static_cast<char *>(p);
+      h->allocs.push_back(p);
+    }
+    (void)cudaGetLastError();
+  }
+  h->oz = h->oz_tc = h->emulated = false;
+  h->Dimg = nullptr;
+  h->Drow = h->Dbal = nullptr;
+  h->capw = nullptr;
+  if (rc == HODLR_OK) rc = alloc_arrays(h, d);
+  if (rc == HODLR_OK && staging) {
+    h->staging = h->alloc<char>(staging, e);
+    if (e != cudaSuccess) rc = set_err(HODLR_ERR_OUT_OF_MEMORY, "staging buffers");
+  }
+  if (rc != HODLR_OK) {
+    free_ctx(h);
+    return rc;
+  }
+  if (one_call) {
+    h->hst = &h->status;
+  } else if (cudaMallocHost(&h->hst, sizeof(DevStatus)) != cudaSuccess) {
+    h->hst = nullptr;
     free_ctx(h);
     return set_err(HODLR_ERR_OUT_OF_MEMORY, "cudaMallocHost");
   }
@@ -1440,6 +1500,16 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
   return HODLR_OK;
 }
 
+static int create_checked(const hodlr_desc *desc, hodlr_handle *out, bool one_call, size_t staging) {
+  if (!desc || !out) return set_err(HODLR_ERR_INVALID_ARG, "null argument");
+  *out = nullptr;
+  const hodlr_desc &d = *desc;
+  if (d.leaf < 1 || d.levels < 0 || d.levels > 24 || d.n != ((int64_t)d.leaf << d.levels))
+    return set_err(HODLR_ERR_INVALID_ARG, "need n = leaf * 2^levels, leaf >= 1, 0 <= levels <= 24");
+  CKS(check_common(d));
+  return create_ctx(d, std::vector<int>(1, d.levels), out, one_call, staging);
+}
+
 // ----------------------------------------------------------------- C ABI
 extern "C" {
 
@@ -1447,15 +1517,7 @@ const char *hodlr_last_error_string(void) { return g_err.c_str(); }
 
 int64_t hodlr_kernel_launches(void) { return (int64_t)g_launches.load(); }
 
-int hodlr_create(const hodlr_desc *desc, hodlr_handle *out) {
-  if (!desc || !out) return set_err(HODLR_ERR_INVALID_ARG, "null argument");
-  *out = nullptr;
-  const hodlr_desc &d = *desc;
-  if (d.leaf < 1 || d.levels < 0 || d.levels > 24 || d.n != ((int64_t)d.leaf << d.levels))
-    return set_err(HODLR_ERR_INVALID_ARG, "need n = leaf * 2^levels, leaf >= 1, 0 <= levels <= 24");
-  CKS(check_common(d));
-  return create_ctx(d, std::vector<int>(1, d.levels), out);
-}
+int hodlr_create(const hodlr_desc *desc, hodlr_handle *out) { return create_checked(desc, out, false, 0); }
 
 int hodlr_destroy(hodlr_handle h) {
   if (!h) return HODLR_OK;
@@ -2060,28 +2122,24 @@ int hodlr_hsolve_ex(int nrow, int nrhs, int rank, int nPart, int LD, double *K, 
   d.refine_tol = 1e-12;
   d.refine_max_iter = 10;
   d.stream = stream;
+  const size_t bk = dev ? 0 : sizeof(double) * nrow * m, bu = dev ? 0 : sizeof(double) * nrow * ucols,
+               bv = dev ? 0 : sizeof(double) * nrow * r;
   hodlr_handle h = nullptr;
-  CKS(hodlr_create(&d, &h));
+  CKS(create_checked(&d, &h, true, bk + bu + bv));
   // K receives the LU factors: leaves up to 128 rows give LU and inverse in one sweep
   h->keep_lu = m <= 128;
   double *dK = K, *dU = U, *dV = V;
   long long ld = LD;
   int rc = HODLR_OK;
-  std::vector<void *> tmp;
   auto fail = [&](int code) {
-    for (void *p : tmp) cudaFree(p);
     hodlr_destroy(h);
     return code;
   };
   if (!dev) {  // stage host buffers through the device, packed (ld = nrow)
     ld = nrow;
-    const size_t bk = sizeof(double) * nrow * m, bu = sizeof(double) * nrow * ucols,
-                 bv = sizeof(double) * nrow * r;
-    dK = dU = dV = nullptr;
-    if (cudaMalloc(&dK, bk) == cudaSuccess) tmp.push_back(dK);
-    if (cudaMalloc(&dU, bu) == cudaSuccess) tmp.push_back(dU);
-    if (cudaMalloc(&dV, bv) == cudaSuccess) tmp.push_back(dV);
-    if (tmp.size() != 3) return fail(set_err(HODLR_ERR_OUT_OF_MEMORY, "hsolve: staging buffers"));
+    dK = reinterpret_cast<double *>(h->staging);
+    dU = reinterpret_cast<double *>(h->staging + bk);
+    dV = reinterpret_cast<double *>(h->staging + bk + bu);
     if (cudaMemcpy2DAsync(dK, sizeof(double) * nrow, K, sizeof(double) * LD, sizeof(double) * nrow, m,
                           cudaMemcpyHostToDevice, h->st) != cudaSuccess ||
         cudaMemcpy2DAsync(dU, sizeof(double) * nrow, U, sizeof(double) * LD, sizeof(double) * nrow, ucols,
