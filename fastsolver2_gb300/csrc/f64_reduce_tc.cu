@@ -13,14 +13,17 @@
 // an SM's share of HBM), the products take 2900 clocks of the tensor pipe; but
 // cutting a value into digits takes some 40 instructions, most of them on the
 // integer pipe, which issues at half rate, and turning the sums into FP64 some
-// 60 an output: 15000 clocks a group measured, the integer pipe 63 % busy.  64
+// 40 an output: 12900 clocks a group measured, the integer pipe two thirds busy.
+// The outputs are rounded on the FP64 pipe (dig_double), which has little else to
+// do here; with the integer packing of dig_value, 60 instructions an output, and
+// the balance held in registers a group took 15000 clocks.  64
 // rows a group because the output side is paid once a group (at 32 rows it
 // would cost as much as the digits), and because 128 would take both of the
 // 57 KB plane buffers that let one half's products overlap the other half's
 // digits.  X's values stay in registers from their load to their digits, and a
 // half's registers are loaded for the next group as soon as they are cut (a
-// first version that loaded the values twice, with eight warps, took 40.3 ms
-// where this one takes 37.0: the reductions of one factor + solve at N = 2^20,
+// first version that loaded the values twice, with eight warps, took 40.3 ms, this
+// order 37.0 at first and now 31.6: the reductions of one factor + solve at N = 2^20,
 // leaf 128, rank 32, 64 right-hand sides.  The FP64 FMA kernel took 229.)
 #include <algorithm>
 
@@ -39,7 +42,7 @@ constexpr long long kWait = 2000000000LL;  // about one second of SM clocks
 struct Shared {
   uint64_t x_full[2], x_empty[2], v_full[2], v_empty[2], bal_full[2], acc_full[2], acc_free[2], drain;
   int xs[4][128], vs[4][kDigN];  // the scales of the last groups
-  unsigned rowmax[4][kGroup];    // largest |V| of each row (high words) of the last groups
+  alignas(16) unsigned rowmax[4][kGroup];    // largest |V| of each row (high words) of the last groups
   unsigned tmem;
   int abort;
 };
@@ -112,6 +115,15 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
   // lanes of a slicer warp: column lane / 8 of four, rows 4 (lane % 8) .. + 3 of each half of the group
   const int lc = lane >> 3, lr = 4 * (lane & 7);
   int g = 0;  // groups this CTA has passed
+  // the balance of four rows of a half of group g (read again for the digits: eight
+  // registers less to hold)
+  auto balance = [&](int g, int h, int *bal) {
+    const uint4 m = *reinterpret_cast<const uint4 *>(&sh->rowmax[g & 3][32 * h + lr]);
+    bal[0] = (int)(m.x >> 20);
+    bal[1] = (int)(m.y >> 20);
+    bal[2] = (int)(m.z >> 20);
+    bal[3] = (int)(m.w >> 20);
+  };
   bool ok = true;
 
   if (warp < kXW) {
@@ -135,20 +147,25 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
     load(w, 0, 0);
     load(w, 0, 1);
     while (u < a.units) {
-      int bal[8], key[2];
+      int key[2] = {kDigZero, kDigZero};
+      unsigned mxs[2] = {0, 0};
       if (!wwait(&sh->bal_full[g & 1], (unsigned)((g >> 1) & 1))) break;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) bal[e] = (int)(sh->rowmax[g & 3][32 * (e >> 2) + lr + (e & 3)] >> 20);
+      for (int h = 0; h < 2; ++h) {
+        int bal[4];
+        balance(g, h, bal);
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const unsigned a = dig_ahi(x[p][4 * h + e]);
+            dig_key(key[p], a, bal[e]);
+            mxs[p] = max(mxs[p], a);
+          }
+      }
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        unsigned mx = 0;
-        key[p] = kDigZero;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const unsigned h = dig_ahi(x[p][e]);
-          dig_key(key[p], h, bal[e]);
-          mx = max(mx, h);
-        }
+        unsigned mx = mxs[p];
 #pragma unroll
         for (int s = 1; s < 8; s <<= 1) {
           key[p] = max(key[p], __shfl_xor_sync(0xffffffffu, key[p], s));
@@ -165,10 +182,12 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
       for (int h = 0; h < 2; ++h) {
         if (g > 0 && !wwait(&sh->x_empty[h], (unsigned)((g - 1) & 1))) ok = false;
         if (!ok) break;
+        int bal[4];
+        balance(g, h, bal);
 #pragma unroll
         for (int p = 0; p < 2; ++p)
           dig_put4(px + h * kDigABytes, kDigAPlane, swz64(4 * warp + lc + 64 * p, lr >> 3) + 2 * (lr & 7), x[p] + 4 * h,
-                   [&](int e) { return bal[4 * h + e]; }, key[p]);
+                   [&](int e) { return bal[e]; }, key[p]);
         fence_proxy_async_smem();
         mbar_arrive(&sh->x_full[h]);
         if (u < a.units) load(w, gi, h);
@@ -216,18 +235,20 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
           ok = false;
           break;
         }
-        int bal[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) bal[e] = -(int)(sh->rowmax[g & 3][32 * (e >> 2) + lr + (e & 3)] >> 20);
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
           int key = kDigZero;
           unsigned mx = 0;
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const unsigned h = dig_ahi(x[p][e]);
-            dig_key(key, h, bal[e]);
-            mx = max(mx, h);
+          for (int h = 0; h < 2; ++h) {
+            int bal[4];
+            balance(g, h, bal);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const unsigned b = dig_ahi(x[p][4 * h + e]);
+              dig_key(key, b, -bal[e]);
+              mx = max(mx, b);
+            }
           }
 #pragma unroll
           for (int s = 1; s < 8; s <<= 1) {
@@ -237,9 +258,12 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
           const int col = 4 * vw + lc + 16 * p;
           if ((lane & 7) == 0) sh->vs[g & 3][col] = dig_scale(key, mx, kDigZeroA);
 #pragma unroll
-          for (int h = 0; h < 2; ++h)
+          for (int h = 0; h < 2; ++h) {
+            int bal[4];
+            balance(g, h, bal);
             dig_put4(pv + (2 * slot + h) * kDigBBytes, kDigBPlane, swz64(col, lr >> 3) + 2 * (lr & 7), x[p] + 4 * h,
-                     [&](int e) { return bal[4 * h + e]; }, key);
+                     [&](int e) { return -bal[e]; }, key);
+          }
         }
         fence_proxy_async_smem();
         mbar_arrive(&sh->v_full[slot]);
@@ -303,13 +327,19 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
           tc_wait_ld(v);
           const int *ev = sh->vs[g & 3] + 16 * h + c2;
           bool odd = false;
-          double y[2];
+          double y[2], f[2];
 #pragma unroll
-          for (int c = 0; c < 2; ++c) y[c] = dig_value(dig_combine<64>(v, c), ex + ev[c], odd);
+          for (int c = 0; c < 2; ++c) {
+            y[c] = dig_double(dig_combine<64>(v, c));
+            f[c] = dig_power(ex + ev[c], odd);
+          }
           if (odd)
-            for (int c = 0; c < 2; ++c) y[c] = dig_value_any(dig_combine<64>(v, c), ex + ev[c]);
-          acc[c2] += y[0];
-          acc[c2 + 1] += y[1];
+            for (int c = 0; c < 2; ++c) {
+              y[c] = dig_value_any(dig_combine<64>(v, c), ex + ev[c]);
+              f[c] = 1.0;
+            }
+          acc[c2] = fma(f[0], y[0], acc[c2]);
+          acc[c2 + 1] = fma(f[1], y[1], acc[c2 + 1]);
         }
         tc_fence_before();
         mbar_arrive(&sh->acc_free[slot]);
