@@ -70,7 +70,7 @@ constexpr int kDigZeroA = 0, kDigZeroB = 2046;  // scales of groups of zeros (an
 
 // |x| as an integer in units of 2^-54 of its group's bound, rounded to
 // nearest, plus 128 in each of its seven low bytes: byte 6 - s of the result
-// is digit s of |x| plus 128.
+// is digit s of |x| plus 128.  Byte 7 is 0x64, the high byte of dig_pair's FP16.
 __device__ __forceinline__ unsigned long long dig_fix(double x, int c, int key) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
   const int e = (int)((hi >> 20) & 0x7ffu);
@@ -79,7 +79,7 @@ __device__ __forceinline__ unsigned long long dig_fix(double x, int c, int key) 
   unsigned long long v;
   const unsigned sh = e ? (unsigned)(key - c - e + 8) : 64u;
   asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(sh));  // shifts past 63 give 0
-  return (v + 0x0101010101010101ull) >> 1;  // (v + 1) / 2, plus 128 in each byte
+  return (v + 0xc901010101010101ull) >> 1;  // (v + 1) / 2 + 0x6480808080808080
 }
 
 // The signs of two values as the factor and addend of dig_pair.
@@ -100,9 +100,11 @@ __device__ __forceinline__ DigSign dig_sign(double x, double y) {
 // the offset: +-(1024 + byte) -+ 1152.
 __device__ __forceinline__ unsigned dig_pair(unsigned long long a, unsigned long long b, const DigSign &sg, int s) {
   const int j = kDig - 1 - s;
-  const unsigned wa = j >= 4 ? (unsigned)(a >> 32) : (unsigned)a, wb = j >= 4 ? (unsigned)(b >> 32) : (unsigned)b;
   const unsigned q = (unsigned)(j & 3);
-  const unsigned t = (__byte_perm(wa, wb, q | (q << 4) | ((q + 4) << 8) | ((q + 4) << 12)) & 0x00ff00ffu) | 0x64006400u;
+  const unsigned t =
+      j >= 4 ? __byte_perm((unsigned)(a >> 32), (unsigned)(b >> 32), q | 0x30u | ((q + 4) << 8) | 0x7000u)
+             : (__byte_perm((unsigned)a, (unsigned)b, q | (q << 4) | ((q + 4) << 8) | ((q + 4) << 12)) & 0x00ff00ffu) |
+                   0x64006400u;
   const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&t), sg.f, sg.a);
   return *reinterpret_cast<const unsigned *>(&r);
 }
