@@ -143,6 +143,7 @@ struct hodlr_ctx {
   // FP64 mode: digit images of the leaf inverses for the tensor-core
   // application, their row scales and balances (null: FMA kernels only)
   unsigned char *Dimg = nullptr;
+  double *gjA = nullptr;  // of a handle for one call: the workspace of a leaf factorisation that keeps LU
   int *Drow = nullptr, *Dbal = nullptr;
   // workspace of the blocked capacitance factorisation (null: one CTA a node):
   // FP64 mode, and mixed mode for ranks above 32 (a 128 x 128 system takes 0.95
@@ -229,7 +230,7 @@ struct hodlr_ctx {
   // One device block holds every array of a small handle: first the sizes are
   // added up (counting), then the arrays laid into it; any other request is an
   // allocation of its own.
-  bool counting = false;
+  bool counting = false, one_call = false;
   size_t block_bytes = 0, block_used = 0;
   char *block = nullptr;
   template <typename T> T *alloc(size_t count, cudaError_t &err) {
@@ -634,7 +635,12 @@ template <typename T> static int factor_sweep(hodlr_ctx *h, bool leaves_done = f
       PHASE(h, HODLR_PHASE_LEAF_LU, launch_mixed_leaf_factor(h, h->dst, s));
     } else if (leaf_inverse_only(h)) {  // LU is the workspace, the images' memory the scratch
       PHASE(h, HODLR_PHASE_LEAF_LU,
-            launch_f64_leaf_gj(h->D, m, (long long)m * m, m, h->nleaf, h->LU, h->ipiv, h->Dinv, h->Dimg, h->dst, s));
+            launch_f64_leaf_gj(h->D, m, (long long)m * m, m, h->nleaf, h->LU, h->ipiv, h->Dinv, nullptr, h->Dimg,
+                               h->dst, s));
+    } else if (sizeof(T) == 8 && h->keep_lu && h->gjA) {
+      PHASE(h, HODLR_PHASE_LEAF_LU,
+            launch_f64_leaf_gj(h->D, m, (long long)m * m, m, h->nleaf, h->gjA, h->ipiv, h->Dinv, h->LU, h->Dimg, h->dst,
+                               s));
     } else {
       PHASE(h, HODLR_PHASE_LEAF_LU,
             launch_leaf_getrf<T>(h->D, m, (long long)m * m, LU, h->ipiv, m, h->nleaf, h->dst, fused ? Dinv : nullptr,
@@ -1365,6 +1371,10 @@ static int alloc_arrays(hodlr_ctx *h, const hodlr_desc &d) {
       if (ie == cudaSuccess) h->Drow = h->alloc<int>(f64_leaf_image_rows(m, h->nleaf), ie);
       if (ie == cudaSuccess) h->Dbal = h->alloc<int>((size_t)n, ie);
       if (ie == cudaSuccess) h->Dimg = img;
+      if (ie == cudaSuccess && h->one_call && m <= 128) {
+        h->gjA = h->alloc<double>((size_t)h->nleaf * m * m, ie);
+        if (ie != cudaSuccess) h->gjA = nullptr;
+      }
     }
     (void)cudaGetLastError();
   }
@@ -1424,6 +1434,7 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
   const long long n = h->n;
   const int L = h->L, r = h->r;
   cudaError_t e = cudaSuccess;
+  h->one_call = one_call;
   h->counting = true;
   int rc = alloc_arrays(h, d);
   if (staging) (void)h->alloc<char>(staging, e);
@@ -1440,6 +1451,7 @@ static int create_ctx(const hodlr_desc &d, const std::vector<int> &sys_levels, h
   h->Dimg = nullptr;
   h->Drow = h->Dbal = nullptr;
   h->capw = nullptr;
+  h->gjA = nullptr;
   if (rc == HODLR_OK) rc = alloc_arrays(h, d);
   if (rc == HODLR_OK && staging) {
     h->staging = h->alloc<char>(staging, e);

@@ -168,12 +168,12 @@ cudaError_t launch_f64_leaf_tc(const unsigned char *img, const int *rows, const 
                                DevStatus *st, cudaStream_t s);
 
 // Dinv = D^-1 of leaves of 64, 128 or 256 rows by blocked Gauss-Jordan, the
-// products on the tensor cores (f64_gj.cu; no LU factors).  A: workspace
-// [nleaf][m][m], ipiv: workspace [nleaf][m]; scratch: f64_leaf_gj_scratch bytes,
+// products on the tensor cores (f64_gj.cu); with LU (m up to 128) the factors and
+// pivots too.  A: workspace [nleaf][m][m], ipiv: [nleaf][m]; scratch: f64_leaf_gj_scratch bytes,
 // 8-byte aligned.
 size_t f64_leaf_gj_scratch(int m, int nleaf);
 cudaError_t launch_f64_leaf_gj(const double *D, long long d_ld, long long d_stride, int m, int nleaf, double *A,
-                               int *ipiv, double *Dinv, void *scratch, DevStatus *st, cudaStream_t s);
+                               int *ipiv, double *Dinv, double *LU, void *scratch, DevStatus *st, cudaStream_t s);
 
 // Capacitance factorisation of the nodes of one depth: S from the T blocks'
 // columns [ucol, ucol + r), FP64 LU (stored in cap_lu / cap_ipiv) and the FP64

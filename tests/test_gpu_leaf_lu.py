@@ -109,3 +109,37 @@ def test_pivots_of_any_magnitude(lib, m):
     x, _ = factored_leaves(lib, D * sc, B * sc)
     exact = np.linalg.solve(D, B.reshape(2, m, 2)).reshape(-1, 2)
     assert np.linalg.norm(x - exact) / np.linalg.norm(exact) <= 4 * m * 2.0 ** -53 * max(map(np.linalg.cond, D)) ** 2
+
+
+@pytest.mark.parametrize("m", [64, 128])
+@pytest.mark.parametrize("npart", [1, 4, 8])
+def test_hsolve_writes_back_the_factors(lib, m, npart):
+    """K's leaves become their LU factors while the inverses are formed: L U has the
+    rows of D in some order, within the componentwise bound of a factorisation of
+    order m, |L| <= 1, and X solves the system."""
+    rng = np.random.default_rng(m + npart)
+    n, r, levels = npart * m, 3, npart.bit_length() - 1
+    D = pivoting_blocks(rng, npart, m)
+    B = rng.standard_normal((n, 2))
+    K = np.asfortranarray(D.reshape(n, m))
+    U = np.asfortranarray(np.hstack([B] + [rng.standard_normal((n, r)) for _ in range(levels)]))
+    V = np.asfortranarray(rng.standard_normal((n, r)) / n)
+    A = np.zeros((n, n))
+    for i in range(npart):
+        A[i * m:(i + 1) * m, i * m:(i + 1) * m] = D[i]
+    for l in range(levels):
+        h = n >> (l + 1)
+        Ul = U[:, 2 + l * r:2 + (l + 1) * r]
+        for q in range(1 << l):
+            c0, c1 = slice(2 * q * h, (2 * q + 1) * h), slice((2 * q + 1) * h, (2 * q + 2) * h)
+            A[c0, c1], A[c1, c0] = Ul[c0] @ V[c1].T, Ul[c1] @ V[c0].T
+    lib.hsolve(n, 2, r, npart, n, K, U, V)
+    assert np.linalg.norm(A @ U[:, :2] - B) <= 8 * n * 2.0 ** -53 * np.linalg.cond(A) ** 2 * np.linalg.norm(B)
+    for i in range(npart):
+        lu = K[i * m:(i + 1) * m]
+        L, R = np.tril(lu, -1) + np.eye(m), np.triu(lu)
+        assert (np.abs(L) <= 1.0 + 2.0 ** -50).all()
+        P = L @ R
+        order = [int(np.argmin(np.abs(D[i] - P[k]).max(axis=1))) for k in range(m)]
+        assert sorted(order) == list(range(m))
+        assert (np.abs(P - D[i][order]) <= 2 * m * 2.0 ** -53 * (np.abs(L) @ np.abs(R))).all()
