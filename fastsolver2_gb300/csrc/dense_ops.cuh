@@ -242,25 +242,61 @@ __device__ void block_laswp(const int *piv, int m, T *X, int ldx, int nc, bool f
 }
 
 // X := A^{-1} X (TRANS = false) or A^{-T} X (TRANS = true) for the LU
-// factors LU (lda) and pivots piv of A, X an m x nc tile (ldx).
-template <typename T, bool TRANS>
+// factors LU (lda) and pivots piv of A, X an m x nc tile (ldx).  FAR (A^{-1}, factors
+// in global memory): a lane's row of a diagonal block is loaded ahead into
+// registers and a row's 32 factors of an update together, instead of one wait of
+// the caches a step.
+template <typename T, bool TRANS, bool FAR = false>
 __device__ void block_getrs(const T *LU, int lda, const int *piv, int m, T *X, int ldx, int nc) {
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
   auto lu = [&](int i, int j) -> T { return LU[i + (long long)j * lda]; };
   if (!TRANS) {
+    T d[FAR ? 32 : 1];
+    auto load_diag = [&](int k0, int kb) {
+#pragma unroll
+      for (int k = 0; k < (FAR ? 32 : 0); ++k) d[k] = lane < kb && k < kb ? lu(k0 + lane, k0 + k) : T(0);
+    };
+    // x_i - sum over the block's rows k of A(i, k) x_k
+    auto row_update = [&](T acc, int i, int k0, int kb, const T *x) {
+      if (FAR) {
+        T l[32];
+#pragma unroll
+        for (int kk = 0; kk < 32; ++kk) l[kk] = kk < kb ? lu(i, k0 + kk) : T(0);
+#pragma unroll
+        for (int kk = 0; kk < 32; ++kk)
+          if (kk < kb) acc -= l[kk] * x[k0 + kk];
+      } else {
+        for (int kk = 0; kk < kb; ++kk) acc -= lu(i, k0 + kk) * x[k0 + kk];
+      }
+      return acc;
+    };
     block_laswp(piv, m, X, ldx, nc, true);
     // L y = P b, L unit lower: 32-row blocks, forward
     for (int k0 = 0; k0 < m; k0 += 32) {
       const int kb = min(32, m - k0);
-      for (int j = warp; j < nc; j += nwarp) {
-        T *x = X + (long long)j * ldx + k0;
-        T v = lane < kb ? x[lane] : T(0);
-        for (int kk = 0; kk < kb - 1; ++kk) {
-          T xk = __shfl_sync(0xffffffffu, v, kk);
-          if (lane > kk && lane < kb) v -= lu(k0 + lane, k0 + kk) * xk;
+      if (FAR) {
+        if (warp < nc) load_diag(k0, kb);
+        for (int j = warp; j < nc; j += nwarp) {
+          T *x = X + (long long)j * ldx + k0;
+          T v = lane < kb ? x[lane] : T(0);
+#pragma unroll
+          for (int kk = 0; kk < 31; ++kk) {
+            const T xk = __shfl_sync(0xffffffffu, v, kk);
+            if (lane > kk && lane < kb) v -= d[kk] * xk;
+          }
+          if (lane < kb) x[lane] = v;
         }
-        if (lane < kb) x[lane] = v;
+      } else {
+        for (int j = warp; j < nc; j += nwarp) {
+          T *x = X + (long long)j * ldx + k0;
+          T v = lane < kb ? x[lane] : T(0);
+          for (int kk = 0; kk < kb - 1; ++kk) {
+            T xk = __shfl_sync(0xffffffffu, v, kk);
+            if (lane > kk && lane < kb) v -= lu(k0 + lane, k0 + kk) * xk;
+          }
+          if (lane < kb) x[lane] = v;
+        }
       }
       __syncthreads();
       const int rows = m - k0 - kb;
@@ -268,9 +304,7 @@ __device__ void block_getrs(const T *LU, int lda, const int *piv, int m, T *X, i
         for (int e = tid; e < rows * nc; e += nt) {
           const int i = k0 + kb + e % rows, j = e / rows;
           T *x = X + (long long)j * ldx;
-          T acc = x[i];
-          for (int kk = 0; kk < kb; ++kk) acc -= lu(i, k0 + kk) * x[k0 + kk];
-          x[i] = acc;
+          x[i] = row_update(x[i], i, k0, kb, x);
         }
       }
       __syncthreads();
@@ -278,24 +312,42 @@ __device__ void block_getrs(const T *LU, int lda, const int *piv, int m, T *X, i
     // U x = y, U non-unit upper: 32-row blocks, backward
     for (int k1 = m; k1 > 0; k1 -= 32) {
       const int k0 = max(0, k1 - 32), kb = k1 - k0;
-      for (int j = warp; j < nc; j += nwarp) {
-        T *x = X + (long long)j * ldx + k0;
-        T v = lane < kb ? x[lane] : T(0);
-        for (int kk = kb - 1; kk >= 0; --kk) {
-          if (lane == kk) v = v / lu(k0 + kk, k0 + kk);
-          T xk = __shfl_sync(0xffffffffu, v, kk);
-          if (lane < kk) v -= lu(k0 + lane, k0 + kk) * xk;
+      if (FAR) {
+        T u = T(1);  // the lane's pivot
+        if (warp < nc) {
+          load_diag(k0, kb);
+          if (lane < kb) u = lu(k0 + lane, k0 + lane);
         }
-        if (lane < kb) x[lane] = v;
+        for (int j = warp; j < nc; j += nwarp) {
+          T *x = X + (long long)j * ldx + k0;
+          T v = lane < kb ? x[lane] : T(0);
+#pragma unroll
+          for (int kk = 31; kk >= 0; --kk) {
+            if (kk >= kb) continue;
+            if (lane == kk) v = v / u;
+            const T xk = __shfl_sync(0xffffffffu, v, kk);
+            if (lane < kk) v -= d[kk] * xk;
+          }
+          if (lane < kb) x[lane] = v;
+        }
+      } else {
+        for (int j = warp; j < nc; j += nwarp) {
+          T *x = X + (long long)j * ldx + k0;
+          T v = lane < kb ? x[lane] : T(0);
+          for (int kk = kb - 1; kk >= 0; --kk) {
+            if (lane == kk) v = v / lu(k0 + kk, k0 + kk);
+            T xk = __shfl_sync(0xffffffffu, v, kk);
+            if (lane < kk) v -= lu(k0 + lane, k0 + kk) * xk;
+          }
+          if (lane < kb) x[lane] = v;
+        }
       }
       __syncthreads();
       if (k0 > 0) {
         for (int e = tid; e < k0 * nc; e += nt) {
           const int i = e % k0, j = e / k0;
           T *x = X + (long long)j * ldx;
-          T acc = x[i];
-          for (int kk = 0; kk < kb; ++kk) acc -= lu(i, k0 + kk) * x[k0 + kk];
-          x[i] = acc;
+          x[i] = row_update(x[i], i, k0, kb, x);
         }
       }
       __syncthreads();

@@ -371,8 +371,8 @@ size_t f64_leaf_gj_scratch(int m, int nleaf) {
 }
 
 // Dinv = D^-1 for every leaf; A: an [nleaf][m][m] workspace, ipiv: [nleaf][m].  With
-// LU (m 64 and 128, not A) the factors and pivots of every leaf as well: hsolve of 8 leaves
-// of 64 rows takes 0.88 ms so, 1.00 with the register-resident sweep.
+// LU (m 64 and 128, not A) the factors and pivots of every leaf as well: hsolve of
+// 8 leaves of 64 rows takes 0.88 ms so, 1.00 with the register-resident sweep.
 cudaError_t launch_f64_leaf_gj(const double *D, long long d_ld, long long d_stride, int m, int nleaf, double *A,
                                int *ipiv, double *Dinv, double *LU, void *scratch, DevStatus *st, cudaStream_t s) {
   double *W = static_cast<double *>(scratch), *R = W + (size_t)nleaf * m * kNb;
