@@ -559,17 +559,18 @@ __global__ void __launch_bounds__(256) update_nn_kernel(UpdateArgs a, int nrt, i
     }
     for (int e = tid; e < BK * kUpdBN; e += 256) {
       const int q = e % BK, j = e / BK;
-      double v = 0.0;
+      T w = T(0);
       if (q0 + q < a.K && j0 + j < a.N) {
-        if (sizeof(T) == 4 && a.B32) {
+        if (sizeof(T) == 4 && a.B32) {  // (by way of FP64 the conversions cost as much as the products)
           const float *B32 = a.B32 + (long long)(b >> 1) * a.b_s1 + (long long)((b & 1) ^ a.b_flip) * a.b_s2;
-          v = a.b_trans ? B32[(j0 + j) + (long long)(q0 + q) * a.ldb] : B32[(q0 + q) + (long long)(j0 + j) * a.ldb];
+          w = a.b_trans ? B32[(j0 + j) + (long long)(q0 + q) * a.ldb] : B32[(q0 + q) + (long long)(j0 + j) * a.ldb];
         } else {
-          v = a.b_trans ? B[(j0 + j) + (long long)(q0 + q) * a.ldb] : B[(q0 + q) + (long long)(j0 + j) * a.ldb];
+          double v = a.b_trans ? B[(j0 + j) + (long long)(q0 + q) * a.ldb] : B[(q0 + q) + (long long)(j0 + j) * a.ldb];
           if (a.scale) v *= a.scale_cols ? a.scale[j0 + j] : a.scale[q0 + q];
+          w = (T)v;
         }
       }
-      sB[q][j] = (T)v;
+      sB[q][j] = w;
     }
     __syncthreads();
 #pragma unroll 4
@@ -796,6 +797,12 @@ cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st)
     HODLR_LAUNCH((update_nn_kernel<T, 32>), (unsigned)nblk, 256, 0, s, a, nrt, nct);
   return cudaGetLastError();
 }
+cudaError_t launch_update_fma_f32(const UpdateArgs &a, cudaStream_t s) {
+  const int nrt = ceil_div(a.M, kUpdBM), nct = ceil_div(a.N, kUpdBN);
+  HODLR_LAUNCH((update_nn_kernel<float, 32>), (unsigned)((long long)nrt * nct * a.nbatch), 256, 0, s, a, nrt, nct);
+  return cudaGetLastError();
+}
+
 template cudaError_t launch_update_nn<double>(const UpdateArgs &, cudaStream_t, DevStatus *);
 template cudaError_t launch_update_nn<float>(const UpdateArgs &, cudaStream_t, DevStatus *);
 

@@ -136,6 +136,7 @@ cudaError_t launch_f64_thin_leaf(const double *Dinv, int m, int nleaf, double *X
                                  const int *skip, cudaStream_t s);
 template <typename T>
 cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st = nullptr);
+cudaError_t launch_update_fma_f32(const UpdateArgs &a, cudaStream_t s);  // FP32 FMAs for any shape
 
 // Explicit inverses of the leaf blocks from their LU factors ([nleaf][m][m]).
 template <typename T>

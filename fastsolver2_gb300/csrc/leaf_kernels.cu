@@ -121,9 +121,14 @@ leaf_getrs_kernel(const T *__restrict__ LU, const int *__restrict__ ipiv, int m,
   }
 }
 
-// Quotients by one divisor, by its reciprocal in two parts: rounded as the division
-// rounds but for extreme exponents, which are left to it.
-struct Quotient {
+// Quotients by one divisor, in FP64 by its reciprocal in two parts: rounded as the
+// division rounds but for extreme exponents, which are left to it.
+template <typename T> struct Quotient {
+  T u;
+  __device__ __forceinline__ static Quotient by(T u) { return Quotient{u}; }
+  __device__ __forceinline__ T of(T x) const { return x / u; }
+};
+template <> struct Quotient<double> {
   double u, hi, lo;
   int ok;
   __device__ __forceinline__ static Quotient by(double u) {
@@ -136,22 +141,24 @@ struct Quotient {
   }
 };
 
-// X := D^{-1} X in FP64 for many columns: 32-row diagonal blocks in launches of
-// their own -- 32 columns a CTA, lane = column, each of the four warps with every
-// fourth row in registers, row k passed through shared memory once it is done, a
-// step a barrier and up to eight FMAs --, the updates of the other rows on the
-// tensor cores (f64_update_tc.cu).  Bound by the FP64 pipe in the diagonal blocks
-// (2 x 496 FMAs a column and block) and by the updates, half each: 2048 leaves of
-// 100 rows, 143 columns and then 5: 5.0 ms, 22.1 with one CTA a leaf and column
-// tile doing it all by FMAs; 512 leaves of 300 rows, 122 columns 4.1 ms, 22.2.
-__global__ void __launch_bounds__(256) leaf_interchange_kernel(const int *__restrict__ ipiv, int m, double *X,
+// X := D^{-1} X for many columns: 32-row diagonal blocks in launches of their own --
+// 32 columns a CTA, lane = column, each of the four warps with every fourth row in
+// registers, row k passed through shared memory once it is done, a step a barrier
+// and up to eight FMAs --, the updates of the other rows in FP64 on the tensor cores
+// (f64_update_tc.cu), in FP32 by FMAs (update_nn_kernel).  FP64 is bound by its pipe
+// in the diagonal blocks (2 x 496 FMAs a column and block) and by the updates, half
+// each: 2048 leaves of 100 rows, 143 columns and then 5: 5.0 ms, 22.1 with one CTA a
+// leaf and column tile doing it all; 512 leaves of 300 rows, 122 columns 4.1 ms,
+// 22.2.  FP32: 1024 leaves of 286 rows, 636 columns and 16 a correction 13.7 ms, 84.
+template <typename T>
+__global__ void __launch_bounds__(256) leaf_interchange_kernel(const int *__restrict__ ipiv, int m, T *X,
                                                                long long ldx, int ncols, int ct, const int *skip) {
   if (skip && *skip) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *sX = reinterpret_cast<double *>(smem_raw);  // [ct][m]
+  T *sX = reinterpret_cast<T *>(smem_raw);  // [ct][m]
   int *sfrom = reinterpret_cast<int *>(sX + (size_t)m * ct), *spiv = sfrom + m;
   const int leaf = blockIdx.y, c0 = blockIdx.x * ct, nc = min(ct, ncols - c0), tid = threadIdx.x;
-  double *Xg = X + (long long)leaf * m + (long long)c0 * ldx;
+  T *Xg = X + (long long)leaf * m + (long long)c0 * ldx;
   for (int i = tid; i < m; i += 256) spiv[i] = ipiv[(long long)leaf * m + i] - 1;
   __syncthreads();
   for (int i = tid; i < m; i += 256) {
@@ -170,28 +177,28 @@ __global__ void __launch_bounds__(256) leaf_interchange_kernel(const int *__rest
       if (sfrom[i] != i) Xg[i + (long long)c * ldx] = sX[c * m + sfrom[i]];
 }
 
-template <bool UPPER>
-__global__ void __launch_bounds__(128) leaf_diag_kernel(const double *__restrict__ LU, int m, int k0, double *X,
+template <typename T, bool UPPER>
+__global__ void __launch_bounds__(128) leaf_diag_kernel(const T *__restrict__ LU, int m, int k0, T *X,
                                                         long long ldx, int ncols, const int *skip) {
   if (skip && *skip) return;
-  __shared__ double sA[32][32], sX[32][33], sK[2][32];  // sA[column][row], sX[column][row]
-  __shared__ Quotient sR[32];
+  __shared__ T sA[32][32], sX[32][33], sK[2][32];  // sA[column][row], sX[column][row]
+  __shared__ Quotient<T> sR[32];
   const int leaf = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kb = min(32, m - k0);
   const int c0 = blockIdx.x * 32;
-  const double *A = LU + (long long)leaf * m * m + k0 + (long long)k0 * m;
-  double *Xg = X + (long long)leaf * m + k0 + (long long)c0 * ldx;
+  const T *A = LU + (long long)leaf * m * m + k0 + (long long)k0 * m;
+  T *Xg = X + (long long)leaf * m + k0 + (long long)c0 * ldx;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int c = warp + 4 * i;
-    sA[c][lane] = lane < kb && c < kb ? A[lane + (long long)c * m] : c == lane ? 1.0 : 0.0;
-    sX[c][lane] = lane < kb && c0 + c < ncols ? Xg[lane + (long long)c * ldx] : 0.0;
+    sA[c][lane] = lane < kb && c < kb ? A[lane + (long long)c * m] : c == lane ? T(1) : T(0);
+    sX[c][lane] = lane < kb && c0 + c < ncols ? Xg[lane + (long long)c * ldx] : T(0);
   }
   __syncthreads();
   if (UPPER) {
-    if (tid < 32) sR[tid] = Quotient::by(sA[tid][tid]);
+    if (tid < 32) sR[tid] = Quotient<T>::by(sA[tid][tid]);
     __syncthreads();
   }
-  double x[8];
+  T x[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) x[q] = sX[lane][4 * q + warp];
 #pragma unroll
@@ -202,7 +209,7 @@ __global__ void __launch_bounds__(128) leaf_diag_kernel(const double *__restrict
       sK[k & 1][lane] = x[k / 4];
     }
     __syncthreads();
-    const double xk = sK[k & 1][lane];
+    const T xk = sK[k & 1][lane];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       if (UPPER ? 4 * q > k : 4 * q + 3 < k) continue;
@@ -223,20 +230,24 @@ __global__ void __launch_bounds__(128) leaf_diag_kernel(const double *__restrict
 // leaf_getrs_kernel, whose time grows with the elements: 16 leaves of 180 rows, 20
 // columns 0.19 ms there and 0.25 here; 32 leaves of 100 rows, 32 columns 0.16 and
 // 0.16; 32 of 180 rows, 70 columns 0.77 and 0.44; 64 of 50 rows, 50 columns 0.19
-// and 0.12.  Up to 8 columns would fill a quarter of a tile: 2048 leaves of 100
-// rows, 5 columns 0.91 and 1.10.
-static bool leaf_getrs_on_tensor_cores(int m, int nleaf, int ncols) {
+// and 0.12.  In FP32, where the one kernel's FMAs cost less, from eight times the
+// elements on: 64 leaves of 100 rows, 83 columns and 11 times 5 0.26 and 0.27 ms, 512
+// of 72 rows, 122 columns 0.56 and 0.36.  Up to 8 columns would fill a quarter of a
+// tile: 2048 leaves of 100 rows, 5 columns 0.91 and 1.10.
+template <typename T> static bool leaf_getrs_by_blocks(int m, int nleaf, int ncols) {
   const char *no_tc = getenv("HODLR_NO_TCGEN05");
-  return !(no_tc && no_tc[0] == '1') && m > 32 && ncols > 8 && (long long)nleaf * ncols * m >= 1 << 17;
+  if (sizeof(T) == 8 && no_tc && no_tc[0] == '1') return false;
+  return m > 32 && m <= 4096 && nleaf <= 65535 && ncols > 8 && (long long)nleaf * ncols * m >= (sizeof(T) == 8 ? 1 << 17 : 1 << 20);
 }
 
-static cudaError_t leaf_getrs_blocked(const double *LU, const int *ipiv, int m, int nleaf, double *X, long long ldx,
+template <typename T>
+static cudaError_t leaf_getrs_blocked(const T *LU, const int *ipiv, int m, int nleaf, T *X, long long ldx,
                                       int ncols, const int *skip, DevStatus *st, cudaStream_t s) {
-  const int ct = std::max(1, std::min(8, (int)(96 * 1024 / ((size_t)m * sizeof(double)))));
-  const size_t bytes = (size_t)m * (ct * sizeof(double) + 2 * sizeof(int));
-  cudaError_t e = allow_dyn_smem(leaf_interchange_kernel, bytes);
+  const int ct = std::max(1, std::min(8, (int)(96 * 1024 / ((size_t)m * sizeof(T)))));
+  const size_t bytes = (size_t)m * (ct * sizeof(T) + 2 * sizeof(int));
+  cudaError_t e = allow_dyn_smem(leaf_interchange_kernel<T>, bytes);
   if (e != cudaSuccess) return e;
-  HODLR_LAUNCH(leaf_interchange_kernel, dim3(ceil_div(ncols, ct), nleaf), 256, bytes, s, ipiv, m, X, ldx, ncols, ct,
+  HODLR_LAUNCH(leaf_interchange_kernel<T>, dim3(ceil_div(ncols, ct), nleaf), 256, bytes, s, ipiv, m, X, ldx, ncols, ct,
                skip);
   const dim3 grid(ceil_div(ncols, 32), nleaf);
   auto update = [&](int k0, int r0, int r1) {  // rows [r0, r1) -= A(rows, block) X(block)
@@ -244,7 +255,10 @@ static cudaError_t leaf_getrs_blocked(const double *LU, const int *ipiv, int m, 
     ua.A = LU + r0 + (long long)k0 * m;
     ua.lda = m;
     ua.a_bstride = (long long)m * m;
-    ua.B = X + k0;
+    if constexpr (sizeof(T) == 8)
+      ua.B = X + k0;
+    else
+      ua.B32 = X + k0;
     ua.ldb = ldx;
     ua.b_s1 = 2LL * m;
     ua.b_s2 = m;
@@ -257,15 +271,16 @@ static cudaError_t leaf_getrs_blocked(const double *LU, const int *ipiv, int m, 
     ua.nbatch = nleaf;
     ua.alpha = -1.0;
     ua.skip = skip;
+    if constexpr (sizeof(T) == 4) return launch_update_fma_f32(ua, s);
     return f64_update_tc_try(ua, st, s, e) ? e : cudaErrorInvalidValue;
   };
   const int last = (m - 1) / 32 * 32;
   for (int k0 = 0; k0 <= last; k0 += 32) {
-    HODLR_LAUNCH(leaf_diag_kernel<false>, grid, 128, 0, s, LU, m, k0, X, ldx, ncols, skip);
+    HODLR_LAUNCH((leaf_diag_kernel<T, false>), grid, 128, 0, s, LU, m, k0, X, ldx, ncols, skip);
     if (k0 < last && (e = update(k0, k0 + 32, m)) != cudaSuccess) return e;
   }
   for (int k0 = last; k0 >= 0; k0 -= 32) {
-    HODLR_LAUNCH(leaf_diag_kernel<true>, grid, 128, 0, s, LU, m, k0, X, ldx, ncols, skip);
+    HODLR_LAUNCH((leaf_diag_kernel<T, true>), grid, 128, 0, s, LU, m, k0, X, ldx, ncols, skip);
     if (k0 > 0 && (e = update(k0, 0, k0)) != cudaSuccess) return e;
   }
   return cudaGetLastError();
@@ -324,9 +339,8 @@ template <typename T>
 cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T *X, long long ldx,
                               int ncols, bool trans, const int *skip, DevStatus *st, cudaStream_t s) {
   if (ncols <= 0 || nleaf <= 0) return cudaSuccess;
-  if constexpr (sizeof(T) == 8)
-    if (!trans && leaf_getrs_on_tensor_cores(m, nleaf, ncols))
-      return leaf_getrs_blocked(LU, ipiv, m, nleaf, X, ldx, ncols, skip, st, s);
+  if (!trans && leaf_getrs_by_blocks<T>(m, nleaf, ncols))
+    return leaf_getrs_blocked<T>(LU, ipiv, m, nleaf, X, ldx, ncols, skip, st, s);
   const size_t lu_bytes = (size_t)m * m * sizeof(T);
   const size_t piv_bytes = (size_t)m * sizeof(int) + 16;
   // FP32: keep two CTAs per SM; FP64 is DFMA-bound, one CTA per SM suffices.

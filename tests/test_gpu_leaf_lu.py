@@ -143,3 +143,15 @@ def test_hsolve_writes_back_the_factors(lib, m, npart):
         order = [int(np.argmin(np.abs(D[i] - P[k]).max(axis=1))) for k in range(m)]
         assert sorted(order) == list(range(m))
         assert (np.abs(P - D[i][order]) <= 2 * m * 2.0 ** -53 * (np.abs(L) @ np.abs(R))).all()
+
+
+@pytest.mark.parametrize("nl,m,k", [(1024, 33, 32), (512, 65, 33), (128, 100, 90), (64, 260, 65)])
+def test_mixed_substitutions_by_blocks(lib, nl, m, k):
+    """FP32 substitutions for many columns: the refined solution within the
+    refinement's tolerance, 1e-12 of the residual, times the condition number."""
+    rng = np.random.default_rng(m)
+    D = pivoting_blocks(rng, nl, m)
+    B = rng.standard_normal((nl * m, k))
+    x, _ = factored_leaves(lib, D, B, mixed=True)
+    exact = np.linalg.solve(D, B.reshape(nl, m, k)).reshape(-1, k)
+    assert np.linalg.norm(x - exact) / np.linalg.norm(exact) <= 2e-12 * max(map(np.linalg.cond, D[:64]))
