@@ -92,8 +92,9 @@ leaf_factor_reg_kernel(const double *__restrict__ D, long long d_ld, long long d
   if (s_info && threadIdx.x == 0) report_error(st, HODLR_ERR_SINGULAR_LEAF, leaf);
 }
 
-template <typename T, bool TRANS, bool LU_SMEM, bool FAR>
-__global__ void __launch_bounds__(256)
+// FAR: block_getrs's, for that many CTAs an SM (0: not).
+template <typename T, bool TRANS, bool LU_SMEM, int FAR>
+__global__ void __launch_bounds__(256, FAR == 2 ? 2 : 0)
 leaf_getrs_kernel(const T *__restrict__ LU, const int *__restrict__ ipiv, int m, T *X, long long ldx,
                   int ncols, int ct, const int *skip) {
   if (skip && *skip) return;
@@ -114,7 +115,7 @@ leaf_getrs_kernel(const T *__restrict__ LU, const int *__restrict__ ipiv, int m,
     sX[e] = Xg[i + (long long)j * ldx];
   }
   __syncthreads();
-  block_getrs<T, TRANS, FAR>(LU_SMEM ? sLU : gLU, m, spiv, m, sX, m, nc);
+  block_getrs<T, TRANS, FAR != 0>(LU_SMEM ? sLU : gLU, m, spiv, m, sX, m, nc);
   for (int e = threadIdx.x; e < m * nc; e += blockDim.x) {
     const int i = e % m, j = e / m;
     Xg[i + (long long)j * ldx] = sX[e];
@@ -352,13 +353,18 @@ cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T 
   // enough column tiles to give every SM a CTA when the leaves are few and large
   int ntile = std::max(ceil_div(ncols, ct_max), std::min(ncols, ceil_div(kNumSMs, nleaf)));
   // Factors far away loaded ahead (block_getrs): in FP32, and in FP64, where that
-  // takes 160 registers a thread, while no SM has two CTAs: one column on each of 4
-  // leaves of 400 rows 0.28 ms, 0.39 without; of 512 leaves of 300 rows 0.86 and 0.53.
-  bool far = !trans && !lu_smem;
+  // takes 160 registers a thread, or 128, while no SM has more than one CTA, or two:
+  // one column on each of 4 leaves of 400 rows 0.28 ms, 0.39 without, of 256 leaves of
+  // 300 rows 0.27 and 0.49, of 512 leaves 0.53 and 0.52.
+  int far = !trans && !lu_smem ? 2 : 0;
   if (far && sizeof(T) == 8) {
     const int nt = std::max(ceil_div(ncols, ct_max), std::min(ncols, std::max(1, kNumSMs / nleaf)));
-    far = (long long)nt * nleaf <= kNumSMs;
-    if (far) ntile = nt;
+    if ((long long)nt * nleaf <= kNumSMs) {
+      far = 1;
+      ntile = nt;
+    } else if ((long long)ntile * nleaf > 2 * kNumSMs) {
+      far = 0;
+    }
   }
   int ct = ceil_div(ncols, ntile);
   ntile = ceil_div(ncols, ct);
@@ -373,11 +379,12 @@ cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T 
     HODLR_LAUNCH(k, grid, 256, bytes, s, LU, ipiv, m, X, ldx, ncols, ct, skip);      \
   }
   if (!trans) {
-    if (lu_smem) HODLR_GETRS_CASE(false, true, false)
-    else if (far) HODLR_GETRS_CASE(false, false, true)
-    else HODLR_GETRS_CASE(false, false, false)
+    if (lu_smem) HODLR_GETRS_CASE(false, true, 0)
+    else if (far == 2) HODLR_GETRS_CASE(false, false, 2)
+    else if (far == 1) HODLR_GETRS_CASE(false, false, 1)
+    else HODLR_GETRS_CASE(false, false, 0)
   } else {
-    if (lu_smem) HODLR_GETRS_CASE(true, true, false) else HODLR_GETRS_CASE(true, false, false)
+    if (lu_smem) HODLR_GETRS_CASE(true, true, 0) else HODLR_GETRS_CASE(true, false, 0)
   }
 #undef HODLR_GETRS_CASE
   return cudaGetLastError();
