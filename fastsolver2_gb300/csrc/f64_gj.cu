@@ -32,7 +32,7 @@
 // 0.6 M for leaf 128 of the 2.1 M of its Gauss-Jordan sweep in one piece.  32
 // columns a block: at 16 the panels would take half as long, but each of twice
 // as many products reads and writes the whole matrix.  Measured with the digit
-// images: 8192 leaves of 128 rows 13.9 ms, 69.7 by the register-resident sweep
+// images: 8192 leaves of 128 rows 13.6 ms, 69.7 by the register-resident sweep
 // (leaf_factor_reg_kernel, at 39 % of the FP64 rate); 16 leaves of 256 rows 1.34
 // ms, 2.50 by blocked LU and triangular solves.  The capacitance systems of N =
 // 2^20, rank 32 (8191 of 64 rows in 13 levels): 6 ms with their applications to

@@ -13,7 +13,7 @@
 // an SM's share of HBM), the products take 2900 clocks of the tensor pipe; but
 // cutting a value into digits takes some 40 instructions, most of them on the
 // integer pipe, which issues at half rate, and turning the sums into FP64 some
-// 40 an output: 12900 clocks a group measured, the integer pipe two thirds busy.
+// 40 an output: 12400 clocks a group measured, the integer pipe two thirds busy.
 // The outputs are rounded on the FP64 pipe (dig_double), which has little else to
 // do here; with the integer packing of dig_value, 60 instructions an output, and
 // the balance held in registers a group took 15000 clocks.  64
@@ -23,7 +23,7 @@
 // digits.  X's values stay in registers from their load to their digits, and a
 // half's registers are loaded for the next group as soon as they are cut (a
 // first version that loaded the values twice, with eight warps, took 40.3 ms, this
-// order 37.0 at first and now 31.6: the reductions of one factor + solve at N = 2^20,
+// order 37.0 at first and now 30.5: the reductions of one factor + solve at N = 2^20,
 // leaf 128, rank 32, 64 right-hand sides.  The FP64 FMA kernel took 229.)
 #include <algorithm>
 
