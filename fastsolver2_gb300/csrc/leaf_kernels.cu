@@ -347,6 +347,14 @@ cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T 
   // FP32: keep two CTAs per SM; FP64 is DFMA-bound, one CTA per SM suffices.
   const size_t cap = sizeof(T) == 4 ? 110 * 1024 : kSmemCap;
   bool lu_smem = lu_bytes + piv_bytes + (size_t)m * 8 * sizeof(T) <= cap;
+  // FP64 factors for up to 8 columns are not worth staging where that leaves an SM
+  // one leaf at a time, or many leaves in turn: 512 leaves of 129 rows, 6 columns 0.38
+  // ms from the caches, 0.55 staged; 2048 of 100 rows, 5 columns 0.75 and 0.91, one
+  // column 0.42 and 0.57; 32 of 100 rows 0.078 and 0.072, 2048 of 50 0.33 both.
+  // Transposed (nothing is loaded ahead there) 64 of 129 rows 0.13 and 0.18, 32 of 150
+  // rows 0.12 and 0.11.
+  if (sizeof(T) == 8 && ncols <= 8 && m >= 64 && ((m > 128 && nleaf >= (trans ? 64 : 1)) || nleaf > 2 * kNumSMs))
+    lu_smem = false;
   size_t avail = cap - piv_bytes - (lu_smem ? lu_bytes : 0);
   int ct_max = (int)std::min<size_t>(avail / ((size_t)m * sizeof(T)), 128);
   if (ct_max < 1) return cudaErrorInvalidValue;

@@ -155,3 +155,20 @@ def test_mixed_substitutions_by_blocks(lib, nl, m, k):
     x, _ = factored_leaves(lib, D, B, mixed=True)
     exact = np.linalg.solve(D, B.reshape(nl, m, k)).reshape(-1, k)
     assert np.linalg.norm(x - exact) / np.linalg.norm(exact) <= 2e-12 * max(map(np.linalg.cond, D[:64]))
+
+
+# factors staged in shared memory or not, by leaf size and number, both ways
+@pytest.mark.parametrize("nl,m", [(512, 64), (512, 63), (256, 100), (32, 129), (64, 129), (2, 165)])
+@pytest.mark.parametrize("k", [1, 8])
+@pytest.mark.parametrize("transpose", [False, True])
+def test_few_columns_staged_or_not(lib, nl, m, k, transpose):
+    rng = np.random.default_rng(nl + m)
+    D = pivoting_blocks(rng, nl, m)
+    B = rng.standard_normal((nl * m, k))
+    _, s = factored_leaves(lib, D, np.ones((nl * m, 8)))
+    b = col(B)
+    s.solve(b, transpose=transpose)
+    A = D.transpose(0, 2, 1) if transpose else D
+    exact = np.linalg.solve(A, B.reshape(nl, m, k)).reshape(-1, k)
+    err = np.linalg.norm(b.cpu().numpy() - exact) / np.linalg.norm(exact)
+    assert err <= 4 * m * 2.0 ** -53 * max(map(np.linalg.cond, D[:64])) ** 2
