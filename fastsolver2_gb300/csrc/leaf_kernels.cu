@@ -360,18 +360,18 @@ cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T 
   if (ct_max < 1) return cudaErrorInvalidValue;
   // enough column tiles to give every SM a CTA when the leaves are few and large
   int ntile = std::max(ceil_div(ncols, ct_max), std::min(ncols, ceil_div(kNumSMs, nleaf)));
-  // Factors far away loaded ahead (block_getrs): in FP32, and in FP64, where that
-  // takes 160 registers a thread, or 128, while no SM has more than one CTA, or two:
-  // one column on each of 4 leaves of 400 rows 0.28 ms, 0.39 without, of 256 leaves of
-  // 300 rows 0.27 and 0.49, of 512 leaves 0.53 and 0.52.
+  // Factors far away loaded ahead (block_getrs) while no SM has more than two CTAs, 128
+  // registers a thread, or in FP64 more than one, 160: one column on each of 4 leaves
+  // of 400 rows 0.28 ms, 0.39 without, of 256 leaves of 300 rows 0.27 and 0.49, of 512
+  // leaves 0.53 and 0.52; in FP32 22 times 2 columns on 1024 leaves of 182 rows 1.7 ms
+  // loaded ahead, 1.4 without.
   int far = !trans && !lu_smem ? 2 : 0;
-  if (far && sizeof(T) == 8) {
+  if (far && (long long)ntile * nleaf > 2 * kNumSMs) far = 0;
+  if (!trans && !lu_smem && sizeof(T) == 8) {
     const int nt = std::max(ceil_div(ncols, ct_max), std::min(ncols, std::max(1, kNumSMs / nleaf)));
     if ((long long)nt * nleaf <= kNumSMs) {
       far = 1;
       ntile = nt;
-    } else if ((long long)ntile * nleaf > 2 * kNumSMs) {
-      far = 0;
     }
   }
   int ct = ceil_div(ncols, ntile);
@@ -389,7 +389,7 @@ cudaError_t launch_leaf_getrs(const T *LU, const int *ipiv, int m, int nleaf, T 
   if (!trans) {
     if (lu_smem) HODLR_GETRS_CASE(false, true, 0)
     else if (far == 2) HODLR_GETRS_CASE(false, false, 2)
-    else if (far == 1) HODLR_GETRS_CASE(false, false, 1)
+    else if (sizeof(T) == 8 && far == 1) HODLR_GETRS_CASE(false, false, 1)
     else HODLR_GETRS_CASE(false, false, 0)
   } else {
     if (lu_smem) HODLR_GETRS_CASE(true, true, 0) else HODLR_GETRS_CASE(true, false, 0)
