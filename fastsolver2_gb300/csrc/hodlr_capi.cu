@@ -1395,7 +1395,7 @@ static int alloc_arrays(hodlr_ctx *h, const hodlr_desc &d) {
 
 // A handle of up to this many bytes takes one allocation: at 2 MB and more a
 // cudaMalloc takes some 50 us and its cudaFree 40, each of the others 1 to 3.
-constexpr size_t kBlockMost = 64u << 20;
+constexpr size_t kBlockMost = size_t(1) << 30;
 
 // Allocate a handle for one tree (sys_levels = {L}) or for a forest of
 // trees with the same leaf size and rank (sys_levels sorted in decreasing
