@@ -1779,22 +1779,27 @@ int hodlr_factor(hodlr_handle h) {
   return factor_end(h);
 }
 
-// Independent handles of one stream factored side by side, handle i's work on
-// streams[i] between two points of `s`.  The first failure is returned, *bad its
-// index; handles after one whose work could not be enqueued are left as they are.
+// Independent handles factored side by side, handle i's work on streams[i] after
+// what its own stream holds.  The first failure is returned, *bad its index; handles
+// after one whose work could not be enqueued are left as they are.
 namespace hodlr {
-int hodlr_factor_many(hodlr_handle *h, int count, cudaStream_t s, const cudaStream_t *streams, cudaEvent_t fork, int *bad) {
-  CK(cudaEventRecord(fork, s));
+int hodlr_factor_many(hodlr_handle *h, int count, const cudaStream_t *streams, cudaEvent_t fork, int *bad) {
+  std::vector<cudaStream_t> own(count);
+  for (int i = 0; i < count; ++i) own[i] = h[i]->st;
   int begun = 0, rc = HODLR_OK;
   for (; begun < count && rc == HODLR_OK; ++begun) {
-    CK(cudaStreamWaitEvent(streams[begun], fork, 0));
+    if (cudaEventRecord(fork, own[begun]) != cudaSuccess ||
+        cudaStreamWaitEvent(streams[begun], fork, 0) != cudaSuccess) {
+      rc = set_err(HODLR_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
+      continue;
+    }
     h[begun]->st = streams[begun];
     rc = factor_begin(h[begun]);
   }
   int first = rc == HODLR_OK ? count : begun - 1;
   std::string why = rc == HODLR_OK ? "" : hodlr_last_error_string();
   for (int i = begun - 1; i >= 0; --i) {
-    if (!(rc != HODLR_OK && i == begun - 1)) {
+    if (rc == HODLR_OK || i != first) {
       const int e = factor_end(h[i]);
       if (e != HODLR_OK) {
         first = i;
@@ -1803,7 +1808,7 @@ int hodlr_factor_many(hodlr_handle *h, int count, cudaStream_t s, const cudaStre
       }
     }
     cudaStreamSynchronize(streams[i]);
-    h[i]->st = s;
+    h[i]->st = own[i];
   }
   *bad = first;
   return rc == HODLR_OK ? rc : set_err(rc, why);

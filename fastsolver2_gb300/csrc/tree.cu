@@ -29,8 +29,8 @@
 
 namespace hodlr {
 
-extern "C" int hodlr_factor_many(hodlr_handle *h, int count, cudaStream_t s, const cudaStream_t *streams, cudaEvent_t fork,
-                           int *bad);  // hodlr_capi.cu
+extern "C" int hodlr_factor_many(hodlr_handle *h, int count, const cudaStream_t *streams, cudaEvent_t fork,
+                                 int *bad);  // hodlr_capi.cu
 
 // One top node of an irregular tree.  T0 = V_c0^T X_c0 is r1 x cols (ld r1),
 // T1 = V_c1^T X_c1 is r0 x cols (ld r0), both in the reduction scratch; the
@@ -532,7 +532,7 @@ int hodlr_tree_factor(hodlr_tree t) {
   std::vector<cudaStream_t> st(t->nsub);
   for (int j = 0; j < t->nsub; ++j) st[j] = t->side[j % t->side.size()];
   int bad = 0;
-  const int frc = hodlr_factor_many(t->sub.data(), t->nsub, t->s, st.data(), t->fork, &bad);
+  const int frc = hodlr_factor_many(t->sub.data(), t->nsub, st.data(), t->fork, &bad);
   if (frc != HODLR_OK)
     return tree_err(frc, std::string("tree_factor: subtree ") + std::to_string(bad) + ": " + hodlr_last_error_string());
   TCK(cudaMemsetAsync(t->dst, 0, sizeof(DevStatus), t->s));

@@ -32,3 +32,23 @@ def test_first_failing_subtree_is_reported(hodlr, top, bad):
         R = tp.B - tp.matvec(to_host(B))
         # backward stable in FP64 on a well-conditioned tree of a few thousand rows
         assert np.linalg.norm(R) / np.linalg.norm(tp.B) < 1e-12
+
+
+def test_subtrees_keep_their_streams(hodlr):
+    """A subtree moved to a stream of the caller's: its inputs set there are seen by
+    the next factorisation, which leaves it on that stream."""
+    shapes = [(64, 2, 4)] * 4
+    tp = P.tree_problem(2, shapes, [3] * 6, nrhs=2, seed=1)
+    t = make_tree(hodlr, tp, nrhs=2)
+    side = torch.cuda.Stream()
+    hodlr.check(hodlr.lib().hodlr_set_stream(t.subtree(1).h, side.cuda_stream))
+    for _ in range(3):
+        with torch.cuda.stream(side):
+            D = to_dev(tp.subs[1].K)
+            t.subtree(1).set_leaf_blocks(D)
+        t.factor()
+        B = to_dev(tp.B)
+        torch.cuda.synchronize()
+        t.solve(B)
+        R = tp.B - tp.matvec(to_host(B))
+        assert np.linalg.norm(R) / np.linalg.norm(tp.B) < 1e-12
