@@ -209,8 +209,11 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
         if (!sync()) break;
         key = max(key, sh->key2[par][half ^ 1][ht]);
         mx = max(mx, sh->mx2[par][half ^ 1][ht]);
-        if (half == 0) sh->ea[rt & 3][ht] = dig_scale(key, mx, kDigZeroA);
         if (ause(rt) > 0 && !wwait(&sh->a_empty[ab], (unsigned)((ause(rt) - 1) & 1))) break;
+        // Only now: the products of row tile rt - 2 (KC 2: rt - 1) are complete, so they
+        // were issued, two tiles after those of rt - 4 at least, once the epilogue had
+        // freed that set -- and read the scales this slot held.
+        if (half == 0) sh->ea[rt & 3][ht] = dig_scale(key, mx, kDigZeroA);
 #pragma unroll
         for (int c = 0; c < KC; ++c)
 #pragma unroll
