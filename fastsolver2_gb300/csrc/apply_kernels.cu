@@ -946,7 +946,7 @@ cudaError_t launch_cap_apply(const CapApplyArgs &a, cudaStream_t s) {
       ua.A = a.sinv + ((long long)a.node_base * n2 + (long long)h * a.r) * n2;
       ua.B = a.Tb + (h ? 0 : a.tb_stride);
       ua.overwrite = h == 0;
-      const cudaError_t e = launch_update_nn<double>(ua, s);
+      const cudaError_t e = launch_update_nn<double>(ua, s, a.st);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

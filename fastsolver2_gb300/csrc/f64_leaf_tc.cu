@@ -32,9 +32,13 @@ constexpr int kAStages = 2, kBStages = 3;
 constexpr int kEpiCols = kDigN * 4 / kEW;  // columns of a set an epilogue thread turns
 constexpr long long kWait = 2000000000LL;  // about one second of SM clocks
 
+__device__ WaitFault g_wait_fault = {-1, -1, 0};
+
 struct Shared {
   uint64_t a_full[kAStages], a_empty[kAStages], b_full[kBStages], b_empty[kBStages], acc_full[2], acc_free[2], drain;
   int eb[4][2 * kDigN];  // the column scales of the last groups
+  long long budget;  // of the wait the hook lets run out, in SM clocks
+  int skip;          // test hook: the stage whose digits are never announced (-1: none)
   unsigned tmem;
   int abort;
 };
@@ -154,6 +158,10 @@ __global__ void __launch_bounds__(kThreads, 1) f64_leaf_tc_kernel(LeafArgs a) {
       mbar_init(&sh->acc_free[q], 32 * kEW);
     }
     mbar_init(&sh->drain, 1);
+    const WaitFault wf = g_wait_fault;
+    const bool hit = wf.cta == (int)blockIdx.x;
+    sh->skip = hit ? wf.stage : -1;
+    sh->budget = hit && wf.budget > 0 ? wf.budget : kWait;
     sh->abort = 0;
     mbar_fence_init();
   }
@@ -247,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1) f64_leaf_tc_kernel(LeafArgs a) {
             dig_put4(pb + slot * Cfg<MT>::kBStage + t * kDigBBytes, kDigBPlane, swz64(col, lr >> 3) + 2 * (lr & 7), x[t],
                      [&](int e) { return e == 0 ? b.x : e == 1 ? b.y : e == 2 ? b.z : b.w; }, key[t]);
           fence_proxy_async_smem();
-          mbar_arrive(&sh->b_full[slot]);
+          if (bs != sh->skip) mbar_arrive(&sh->b_full[slot]);
           if (c + 1 < kc) load(c + 1);
         }
       }
@@ -276,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) f64_leaf_tc_kernel(LeafArgs a) {
         for (int h = 0; ok && h < KH; ++h, ++grp)
           for (int c = 0; ok && c < kc; ++c, ++bs) {
             const int bslot = bs % kBStages;
-            if (!wait(&sh->b_full[bslot], (unsigned)((bs / kBStages) & 1))) ok = false;
+            if (!mbar_wait_or_abort(&sh->b_full[bslot], (unsigned)((bs / kBStages) & 1), &sh->abort, &sh->budget)) ok = false;
             for (int t = 0; ok && t < MT; ++t, ++as) {
               const int aslot = as % kAStages;
               if (!wait(&sh->a_full[aslot], (unsigned)((as / kAStages) & 1))) {
@@ -373,6 +381,10 @@ __global__ void __launch_bounds__(kThreads, 1) f64_leaf_tc_kernel(LeafArgs a) {
     tc_fence_after();
     tc_dealloc(tmem, 2 * kDigAccCols);
   }
+}
+
+cudaError_t f64_leaf_tc_set_wait_fault(const WaitFault &wf) {
+  return cudaMemcpyToSymbol(g_wait_fault, &wf, sizeof wf);
 }
 
 // Sizes of the digit images of nleaf inverses: bytes of planes, ints of row

@@ -39,10 +39,14 @@ constexpr int kMmaWarp = kXW + kVW + kEW, kThreads = 32 * (kMmaWarp + 1);
 constexpr int kGroup = 64;  // rows a group
 constexpr long long kWait = 2000000000LL;  // about one second of SM clocks
 
+__device__ WaitFault g_wait_fault = {-1, -1, 0};
+
 struct Shared {
   uint64_t x_full[2], x_empty[2], v_full[2], v_empty[2], bal_full[2], acc_full[2], acc_free[2], drain;
   int xs[4][128], vs[4][kDigN];  // the scales of the last groups
   alignas(16) unsigned rowmax[4][kGroup];    // largest |V| of each row (high words) of the last groups
+  long long budget;  // of the wait the hook lets run out, in SM clocks
+  int skip;          // test hook: the stage whose digits are never announced (-1: none)
   unsigned tmem;
   int abort;
 };
@@ -98,6 +102,10 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
       mbar_init(&sh->acc_free[q], 32 * kEW);
     }
     mbar_init(&sh->drain, 1);
+    const WaitFault wf = g_wait_fault;
+    const bool hit = wf.cta == (int)blockIdx.x;
+    sh->skip = hit ? wf.stage : -1;
+    sh->budget = hit && wf.budget > 0 ? wf.budget : kWait;
     sh->abort = 0;
     mbar_fence_init();
   }
@@ -266,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
           }
         }
         fence_proxy_async_smem();
-        mbar_arrive(&sh->v_full[slot]);
+        if (g != sh->skip) mbar_arrive(&sh->v_full[slot]);
       }
     }
   } else if (warp == kMmaWarp) {
@@ -276,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
         const Unit w = unit_of(a, u);
         for (int gi = 0; ok && gi < w.groups; ++gi, ++g) {
           const int slot = g & 1;
-          if (!wait(&sh->v_full[slot], (unsigned)((g >> 1) & 1)) ||
+          if (!mbar_wait_or_abort(&sh->v_full[slot], (unsigned)((g >> 1) & 1), &sh->abort, &sh->budget) ||
               (g >= 2 && !wait(&sh->acc_free[slot], (unsigned)(((g >> 1) - 1) & 1)))) {
             ok = false;
             break;
@@ -381,6 +389,10 @@ void f64_reduce_tc_plan(long long nrows, int nbatch, int r, int C, int per_sm, i
     nchunks = (int)m;
     chunk_rows = (int)std::min<long long>(rows, nrows);
   }
+}
+
+cudaError_t f64_reduce_tc_set_wait_fault(const WaitFault &wf) {
+  return cudaMemcpyToSymbol(g_wait_fault, &wf, sizeof wf);
 }
 
 bool f64_reduce_tc_try(const double *V, long long ldv, const double *X, long long ldx, long long nrows, int nbatch,

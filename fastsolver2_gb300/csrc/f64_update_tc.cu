@@ -34,12 +34,16 @@ constexpr int kEpiCols = kDigN * 128 / kEpi;  // columns of an epilogue thread
 constexpr int kMmaWarp = (kSlicers + kEpi) / 32;
 constexpr long long kWait = 2000000000LL;  // about one second of SM clocks
 
+__device__ WaitFault g_wait_fault = {-1, -1, 0};
+
 struct Shared {
   uint64_t a_full[2], a_empty[2], b_full[2], b_empty[2], acc_full[2], acc_free[2], slicers, drain;
   int ea[4][128], eb[8][kDigN];  // the scales of the last row tiles and tiles, read by the epilogue
   unsigned colw[2][4][64];       // largest |A(., k)| of each 32 rows of the last row tiles (high words)
   int key2[2][2][128];           // each half's key and largest of a row, of the last row tiles
   unsigned mx2[2][2][128];
+  long long budget;  // of the wait the hook lets run out, in SM clocks
+  int skip;          // test hook: the stage whose digits are never announced (-1: none)
   unsigned tmem;
   int abort;
 };
@@ -94,6 +98,10 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
     }
     mbar_init(&sh->slicers, kSlicers);
     mbar_init(&sh->drain, 1);
+    const WaitFault wf = g_wait_fault;
+    const bool hit = wf.cta == (int)blockIdx.x;
+    sh->skip = hit ? wf.stage : -1;
+    sh->budget = hit && wf.budget > 0 ? wf.budget : kWait;
     sh->abort = 0;
     mbar_fence_init();
   }
@@ -269,7 +277,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
                    [&](int e) { return bx[e]; }, key);
       }
       fence_proxy_async_smem();
-      mbar_arrive(&sh->b_full[slot]);
+      if (ti != sh->skip) mbar_arrive(&sh->b_full[slot]);
       wb.next();
       wb.next();
       if (wb.t < t1) load_b(wb);
@@ -280,7 +288,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
       for (Walk w(nrt, nct, t0); w.t < t1; w.next()) {
         const int ti = w.t - t0, rt = w.rt, ab = abuf(rt), slot = ti & 1;
         if ((w.t == t0 || w.ct == 0) && !wait(&sh->a_full[ab], (unsigned)(ause(rt) & 1))) break;
-        if (!wait(&sh->b_full[slot], (unsigned)((ti >> 1) & 1)) ||
+        if (!mbar_wait_or_abort(&sh->b_full[slot], (unsigned)((ti >> 1) & 1), &sh->abort, &sh->budget) ||
             (ti >= 2 && !wait(&sh->acc_free[slot], (unsigned)(((ti >> 1) - 1) & 1))))
           break;
         tc_fence_after();
@@ -371,6 +379,10 @@ static cudaError_t launch_kc(const UpdateArgs &a, DevStatus *st, cudaStream_t s)
   const int ntiles = nrt * nct * a.nbatch;
   HODLR_LAUNCH(k, (unsigned)std::min(ntiles, kNumSMs), kThreads, Cfg<KC>::kSmem, s, a, nrt, nct, ntiles, st);
   return cudaGetLastError();
+}
+
+cudaError_t f64_update_tc_set_wait_fault(const WaitFault &wf) {
+  return cudaMemcpyToSymbol(g_wait_fault, &wf, sizeof wf);
 }
 
 bool f64_update_tc_try(const UpdateArgs &a, DevStatus *st, cudaStream_t s, cudaError_t &err) {

@@ -814,6 +814,9 @@ extern "C" int hodlr_debug_wait_fault(int cta, int stage, long long budget_cycle
   const hodlr::WaitFault wf = {cta, cta < 0 ? -1 : stage, cta < 0 ? 0 : budget_cycles};
   cudaError_t e = cudaMemcpyToSymbol(hodlr::g_wait_fault, &wf, sizeof wf);
   if (e == cudaSuccess) e = hodlr::reduce_tc_set_wait_fault(wf);
+  if (e == cudaSuccess) e = hodlr::f64_update_tc_set_wait_fault(wf);
+  if (e == cudaSuccess) e = hodlr::f64_reduce_tc_set_wait_fault(wf);
+  if (e == cudaSuccess) e = hodlr::f64_leaf_tc_set_wait_fault(wf);
   if (e != cudaSuccess) return hodlr::set_last_error(HODLR_ERR_CUDA, cudaGetErrorString(e));
   return HODLR_OK;
 }

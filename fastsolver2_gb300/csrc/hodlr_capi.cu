@@ -555,6 +555,7 @@ static int cap_apply(hodlr_ctx *h, int l, int C, long long tb_stride, bool trans
   ca.node_base = h->node_base(l);
   ca.trans = trans;
   ca.skip = skip;
+  ca.st = h->dst;
   PHASE(h, HODLR_PHASE_CAPACITANCE, launch_cap_apply(ca, h->st));
   return HODLR_OK;
 }
@@ -795,13 +796,14 @@ static int matvec_fp64(hodlr_ctx *h, bool trans, const double *X, long long ldx,
   la.nbatch = h->nleaf;
   la.alpha = alpha;
   la.skip = skip;
-  PHASE(h, HODLR_PHASE_RESID_LEAF, launch_update_nn<double>(la, s));
+  PHASE(h, HODLR_PHASE_RESID_LEAF, launch_update_nn<double>(la, s, h->dst));
   for (int l = 0; l < L; ++l) {
     const int nb = h->nb(l);
     const long long rows = h->rows(l);
     const double *Ared = trans ? h->Ulev(l) : h->Vlev(l);
     const double *Aupd = trans ? h->Vlev(l) : h->Ulev(l);
-    PHASE(h, HODLR_PHASE_RESID_REDUCE, launch_reduce_tn<double>(Ared, n, X, ldx, rows, nb, r, k, h->Tbuf, h->red, skip, s));
+    PHASE(h, HODLR_PHASE_RESID_REDUCE,
+          launch_reduce_tn<double>(Ared, n, X, ldx, rows, nb, r, k, h->Tbuf, h->red, skip, s, h->dst));
     UpdateArgs ua{};
     ua.A = Aupd;
     ua.lda = n;
@@ -821,7 +823,7 @@ static int matvec_fp64(hodlr_ctx *h, bool trans, const double *X, long long ldx,
     ua.nbatch = nb;
     ua.alpha = alpha;
     ua.skip = skip;
-    PHASE(h, HODLR_PHASE_RESID_UPDATE, launch_update_nn<double>(ua, s));
+    PHASE(h, HODLR_PHASE_RESID_UPDATE, launch_update_nn<double>(ua, s, h->dst));
   }
   return HODLR_OK;
 }
@@ -1923,13 +1925,13 @@ int hodlr_adjoint(hodlr_handle h, const double *x, int64_t ldx, const double *g,
     ua.K = k;
     ua.nbatch = h->nleaf;
     ua.alpha = -1.0;
-    CK(launch_update_nn<double>(ua, s));
+    CK(launch_update_nn<double>(ua, s, h->dst));
   }
   for (int l = 0; l < L && (gr->dU || gr->dV || gr->ds); ++l) {
     const int nb = h->nb(l);
     const long long rows = h->rows(l);
-    CK(launch_reduce_tn<double>(h->Vlev(l), n, x, ldx, rows, nb, r, k, h->Tbuf, h->red, nullptr, s));
-    CK(launch_reduce_tn<double>(h->Ulev(l), n, lam, ldl, rows, nb, r, k, h->Wbuf, h->red, nullptr, s));
+    CK(launch_reduce_tn<double>(h->Vlev(l), n, x, ldx, rows, nb, r, k, h->Tbuf, h->red, nullptr, s, h->dst));
+    CK(launch_reduce_tn<double>(h->Ulev(l), n, lam, ldl, rows, nb, r, k, h->Wbuf, h->red, nullptr, s, h->dst));
     for (int which = 0; which < 2; ++which) {
       double *dst = which == 0 ? gr->dU : gr->dV;
       if (!dst) continue;
@@ -1956,7 +1958,7 @@ int hodlr_adjoint(hodlr_handle h, const double *x, int64_t ldx, const double *g,
       ua.K = k;
       ua.nbatch = nb;
       ua.alpha = -1.0;
-      CK(launch_update_nn<double>(ua, s));
+      CK(launch_update_nn<double>(ua, s, h->dst));
     }
     if (gr->ds) CK(launch_scale_grad(h->Wbuf, h->Tbuf, r, k, nb, gr->ds + (long long)l * r, s));
   }
@@ -2067,7 +2069,7 @@ int hodlr_generate(hodlr_handle h, uint64_t seed, double shift, int orthonormal,
       CK(launch_gaussian(X, n, n, r, seed, stream, orthonormal ? 1.0 : 1.0 / std::sqrt((double)rows), s));
       if (!orthonormal) continue;
       for (int pass = 0; pass < 2; ++pass) {  // CholeskyQR2 per child block
-        CK(launch_reduce_tn<double>(X, n, X, n, rows, nb, r, r, h->Tbuf, h->red, nullptr, s));
+        CK(launch_reduce_tn<double>(X, n, X, n, rows, nb, r, r, h->Tbuf, h->red, nullptr, s, h->dst));
         CK(launch_chol_inv(h->Tbuf, h->eta, r, nb, h->dst, s));
         CK(cudaMemsetAsync(tmp, 0, sizeof(double) * n * r, s));
         UpdateArgs ua{};
@@ -2086,7 +2088,7 @@ int hodlr_generate(hodlr_handle h, uint64_t seed, double shift, int orthonormal,
         ua.K = r;
         ua.nbatch = nb;
         ua.alpha = 1.0;
-        CK(launch_update_nn<double>(ua, s));
+        CK(launch_update_nn<double>(ua, s, h->dst));
         CK(cudaMemcpyAsync(X, tmp, sizeof(double) * n * r, cudaMemcpyDeviceToDevice, s));
       }
     }
@@ -2370,7 +2372,7 @@ int hodlr_set_seeded(hodlr_handle h, const int64_t *useeds, const int64_t *vseed
 
 int hodlr_set_uvd(hodlr_handle h, const double *U, int64_t ldu, const double *V, int64_t ldv, const double *Dg) {
   if (!h || !U || !V || !Dg) return set_err(HODLR_ERR_INVALID_ARG, "null argument");
-  CKS(join_prep(h));  // the inputs are rewritten: set-time preparation still reading them ends first
+  CKS(reset_status(h));  // (the inputs are rewritten: set-time preparation still reading them ends first)
   if (ldu < h->n || ldv < h->n) return set_err(HODLR_ERR_INVALID_ARG, "ld < n");
   std::fill(h->vsrc.begin(), h->vsrc.end(), nullptr);
   const long long n = h->n;
@@ -2409,7 +2411,7 @@ int hodlr_set_uvd(hodlr_handle h, const double *U, int64_t ldu, const double *V,
   ua.K = r;
   ua.nbatch = h->nleaf;
   ua.alpha = 1.0;
-  CK(launch_update_nn<double>(ua, s));
+  CK(launch_update_nn<double>(ua, s, h->dst));
   CK(launch_add_leaf_diag(h->D, dD, m, h->nleaf, s));
   CK(cudaFreeAsync(dD, s));
   for (int l = 0; l < L; ++l) {
@@ -2420,8 +2422,7 @@ int hodlr_set_uvd(hodlr_handle h, const double *U, int64_t ldu, const double *V,
   h->leaves_prefactored = false;
   CKS(prepare_leaves(h));
   h->factored = false;
-  CK(cudaStreamSynchronize(s));
-  return HODLR_OK;
+  return sync_status(h, nullptr);
 }
 
 }  // extern "C"
@@ -2450,15 +2451,16 @@ int hodlr_gemm_reduce(int nrow, int nPart, int ncolV, int ncolU, const double *V
     return set_err(HODLR_ERR_INVALID_ARG, "gemm_reduce: bad arguments");
   const long long rows = nrow / nPart;
   Scratch sc;
+  CallStatus st;
+  CK(st.find());
   double *out = sc.get<double>((size_t)nPart * ncolV * ncolU);
   double *work = sc.get<double>(reduce_workspace_doubles(rows, nPart, ncolV, ncolU, 8));
   if (!out || !work) return set_err(HODLR_ERR_OUT_OF_MEMORY, "gemm_reduce: scratch");
-  CK(launch_reduce_tn<double>(V, ldv, U, ldu, rows, nPart, ncolV, ncolU, out, work, nullptr, 0));
+  CK(launch_reduce_tn<double>(V, ldv, U, ldu, rows, nPart, ncolV, ncolU, out, work, nullptr, 0, st.word()));
   for (int p = 0; p < nPart; ++p)  // block p (ncolV x ncolU, ld ncolV) -> rows p*ncolV of W
     CK(cudaMemcpy2DAsync(W + (long long)p * ncolV, sizeof(double) * ldw, out + (long long)p * ncolV * ncolU,
                          sizeof(double) * ncolV, sizeof(double) * ncolV, ncolU, cudaMemcpyDeviceToDevice, 0));
-  CK(cudaStreamSynchronize(0));
-  return HODLR_OK;
+  return st.finish("gemm_reduce");
 }
 
 int hodlr_gemm_broadcast(int nrow, int nPart, int nBlock, int K, int N, double alpha, const double *U, int64_t ldu,
@@ -2468,6 +2470,8 @@ int hodlr_gemm_broadcast(int nrow, int nPart, int nBlock, int K, int N, double a
     return set_err(HODLR_ERR_INVALID_ARG, "gemm_broadcast: bad arguments");
   const long long rows = nrow / nPart;
   const int per = nPart / nBlock;  // row partitions sharing one block of Vb
+  CallStatus st;
+  CK(st.find());
   if (beta != 1.0) CK(launch_axpy(W, ldw, W, ldw, nrow, N, beta, false, nullptr, 0));
   for (int blk = 0; blk < nBlock; ++blk) {
     UpdateArgs ua{};
@@ -2484,10 +2488,9 @@ int hodlr_gemm_broadcast(int nrow, int nPart, int nBlock, int K, int N, double a
     ua.K = K;
     ua.nbatch = per;
     ua.alpha = alpha;
-    CK(launch_update_nn<double>(ua, 0));
+    CK(launch_update_nn<double>(ua, 0, st.word()));
   }
-  CK(cudaStreamSynchronize(0));
-  return HODLR_OK;
+  return st.finish("gemm_broadcast");
 }
 
 int hodlr_node_solve(int nnode, int r, int nrhs, const double *VTu, int64_t ldu, double *VTd, int64_t ldd) {
@@ -2530,12 +2533,14 @@ int hodlr_node_solve(int nnode, int r, int nrhs, const double *VTu, int64_t ldu,
   ca.r = r;
   ca.C = nrhs;
   ca.nnode = nnode;
+  ca.st = st;
   CK(launch_cap_apply(ca, 0));
   for (int p = 0; p < nnode; ++p)  // eta_p (2r x nrhs, ld 2r) -> rows [2r p, 2r (p+1)) of VTd
     CK(cudaMemcpy2DAsync(VTd + (long long)p * 2 * r, sizeof(double) * ldd, eta + (long long)p * 2 * r * nrhs,
                          sizeof(double) * 2 * r, sizeof(double) * 2 * r, nrhs, cudaMemcpyDeviceToDevice, 0));
   DevStatus hs{};
   CK(cudaMemcpy(&hs, st, sizeof(DevStatus), cudaMemcpyDeviceToHost));
+  if (hs.code == HODLR_ERR_TIMEOUT) return set_err(hs.code, "node_solve: device wait timed out (index " + std::to_string(hs.index) + ")");
   if (hs.code) return set_err(hs.code, "node_solve: singular capacitance system");
   return HODLR_OK;
 }

@@ -10,6 +10,25 @@ namespace hodlr {
 // Record the message returned by hodlr_last_error_string(); returns code.
 int set_last_error(int code, const char *msg);
 
+// The status word of a call that has no handle, on the legacy default stream of
+// the current device: one of a fixed set of device words (component_status.cu),
+// taken for the lifetime of the object; with all of them taken by other threads'
+// calls, construction waits for one.
+class CallStatus {
+ public:
+  CallStatus();
+  ~CallStatus();
+  CallStatus(const CallStatus &) = delete;
+  CallStatus &operator=(const CallStatus &) = delete;
+  cudaError_t find();  // before word()
+  DevStatus *word() const { return word_; }
+  int finish(const char *call);  // waits for the stream; the call's status, with the error's text set
+
+ private:
+  DevStatus *word_ = nullptr;
+  int slot_;
+};
+
 // Launch-shape choices of the tunable kernels, chosen per handle (per forest
 // of a batch) by the autotuner.  Launches made by a host thread use the
 // choices of the innermost live TuningScope on that thread (defaults
@@ -92,7 +111,9 @@ bool reduce_tc_try(const float *V, long long ldv, const float *X, long long ldx,
 
 // Test hook of the bounded waits (set by hodlr_debug_wait_fault, off in
 // normal use): CTA `cta` of every launch of the FP32 row-reduction kernels
-// does not issue the copies of its stage `stage`, so nothing ever completes
+// does not issue the copies of its stage `stage`, and of the FP64 digit-product
+// kernels (f64_update_tc.cu, f64_reduce_tc.cu, f64_leaf_tc.cu) does not announce
+// the digits of its tile, row group or chunk `stage`, so nothing ever completes
 // that stage's mbarrier phase and the CTA's wait on it can only end by its
 // clock budget, `budget` cycles for that CTA (0 = the default budget; every
 // other CTA keeps the default).  Each kernel's file holds its own device copy.
@@ -101,6 +122,9 @@ struct WaitFault {
   long long budget;
 };
 cudaError_t reduce_tc_set_wait_fault(const WaitFault &wf);
+cudaError_t f64_update_tc_set_wait_fault(const WaitFault &wf);
+cudaError_t f64_reduce_tc_set_wait_fault(const WaitFault &wf);
+cudaError_t f64_leaf_tc_set_wait_fault(const WaitFault &wf);
 template <typename T>
 cudaError_t launch_reduce_tn(const T *A, long long lda, const T *X, long long ldx, long long nrows,
                              int nbatch, int r, int C, double *out, double *work, const int *skip,
@@ -212,6 +236,7 @@ struct CapApplyArgs {
   int r, C, nnode, node_base;
   bool trans;
   const int *skip;
+  DevStatus *st;  // of the tensor-core products' waits
 };
 cudaError_t launch_cap_apply(const CapApplyArgs &a, cudaStream_t s);
 cudaError_t launch_f64_thin_cap(const CapApplyArgs &a, cudaStream_t s);  // FP64, up to 8 columns

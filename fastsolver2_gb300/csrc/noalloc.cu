@@ -75,16 +75,17 @@ extern "C" int hodlr_gemm_reduce_noalloc(int nrow, int nPart, int ncolV, int nco
   double *scratch = nullptr;
   int st = scratch_address(&scratch);
   if (st != HODLR_OK) return st;
+  CallStatus status;
+  cudaError_t e = status.find();
+  if (e != cudaSuccess) return set_last_error(HODLR_ERR_CUDA, cudaGetErrorString(e));
   double *out = scratch;            // per-partition blocks, ncolV x ncolU each
   double *partial = scratch + blocks;  // split-K partial sums (written before read)
-  cudaError_t e = launch_reduce_tn<double>(V, ldv, U, ldu, rows, nPart, ncolV, ncolU, out, partial, nullptr, 0);
+  e = launch_reduce_tn<double>(V, ldv, U, ldu, rows, nPart, ncolV, ncolU, out, partial, nullptr, 0, status.word());
   if (e != cudaSuccess) return set_last_error(HODLR_ERR_CUDA, cudaGetErrorString(e));
   for (int p = 0; p < nPart; ++p) {  // block p -> rows p*ncolV of W (a copy, not an allocation)
     e = cudaMemcpy2DAsync(W + (long long)p * ncolV, sizeof(double) * ldw, out + (size_t)p * ncolV * ncolU,
                           sizeof(double) * ncolV, sizeof(double) * ncolV, ncolU, cudaMemcpyDeviceToDevice, 0);
     if (e != cudaSuccess) return set_last_error(HODLR_ERR_CUDA, cudaGetErrorString(e));
   }
-  e = cudaStreamSynchronize(0);
-  if (e != cudaSuccess) return set_last_error(HODLR_ERR_CUDA, cudaGetErrorString(e));
-  return HODLR_OK;
+  return status.finish("gemm_reduce_noalloc");
 }

@@ -132,6 +132,19 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t *bar, unsigned parit
   }
   return true;
 }
+// The same with the limit in shared memory, read only by a wait that has to spin.
+__device__ __forceinline__ bool mbar_wait_or_abort(uint64_t *bar, unsigned parity, int *abort, const long long *limit) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*(volatile int *)abort) return false;
+    if (clock64() - t0 > *(const volatile long long *)limit) {
+      *(volatile int *)abort = 1;
+      return false;
+    }
+  }
+  return true;
+}
 
 // Exact three-way bf16 split of two FP32 values, x = h + m + l (24
 // significant bits; both subtractions are exact), for FP32-class products on

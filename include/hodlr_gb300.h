@@ -495,7 +495,9 @@ HODLR_API int hodlr_tree_matvec(hodlr_tree t, const double *X, int64_t ldx, doub
  * whose CPU tasks have no device waits).  While set (cta >= 0), CTA `cta` of
  * every launch of the FP32 row-reduction kernels (the TMA-fed V^T X of the
  * mixed path, on the tensor cores or on the FMA pipe) does not issue the
- * copies of its stage `stage` (counted over the CTA's launch), so its wait on
+ * copies of its stage `stage` (counted over the CTA's launch), and of the FP64
+ * tensor-core kernels (low-rank update, row reduction, leaf application) does
+ * not announce the digits of its tile, row group or chunk `stage`, so its wait on
  * that stage ends only by a clock budget of `budget_cycles` SM cycles
  * (1 .. 1e9; 0 = the default of 1e9): the CTA records HODLR_ERR_TIMEOUT with
  * its index in the handle's status word, waits (bounded) for its copies in
