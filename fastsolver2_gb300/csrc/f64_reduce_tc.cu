@@ -41,17 +41,6 @@ constexpr long long kWait = 2000000000LL;  // about one second of SM clocks
 
 __device__ WaitFault g_wait_fault = {-1, -1, 0};
 
-struct Shared {
-  uint64_t x_full[2], x_empty[2], v_full[2], v_empty[2], bal_full[2], acc_full[2], acc_free[2], drain;
-  int xs[4][128], vs[4][kDigN];  // the scales of the last groups
-  alignas(16) unsigned rowmax[4][kGroup];    // largest |V| of each row (high words) of the last groups
-  long long budget;  // of the wait the hook lets run out, in SM clocks
-  int skip;          // test hook: the stage whose digits are never announced (-1: none)
-  unsigned tmem;
-  int abort;
-};
-constexpr size_t kSmem = (size_t)2 * kDigABytes + (size_t)4 * kDigBBytes + sizeof(Shared) + 1024;
-
 struct RedArgs {
   const double *V, *X;
   long long ldv, ldx, nrows;
@@ -61,6 +50,19 @@ struct RedArgs {
   const int *skip;
   DevStatus *st;
 };
+
+struct Shared {
+  uint64_t x_full[2], x_empty[2], v_full[2], v_empty[2], bal_full[2], acc_full[2], acc_free[2], drain;
+  int xs[4][128], vs[4][kDigN];  // the scales of the last groups
+  alignas(16) unsigned rowmax[4][kGroup];    // largest |V| of each row (high words) of the last groups
+  long long budget;  // of the wait the hook lets run out, in SM clocks
+  int skip;          // test hook: the stage whose digits are never announced (-1: none)
+  unsigned tmem;
+  int marked;    // a result is a NaN
+  RedArgs args;  // for sum_marked (the address of a kernel's parameter costs registers)
+  int abort;
+};
+constexpr size_t kSmem = (size_t)2 * kDigABytes + (size_t)4 * kDigBBytes + sizeof(Shared) + 1024;
 
 struct Unit {
   long long row0, blk;  // first row; index of the r x C result
@@ -79,6 +81,25 @@ __device__ __forceinline__ Unit unit_of(const RedArgs &a, long long u) {
   w.rows = (int)min((long long)a.chunk_rows, a.nrows - r0);
   w.groups = (w.rows + kGroup - 1) / kGroup;
   return w;
+}
+
+// The results of a CTA's units that are NaN -- an infinity or NaN among their values
+// -- again by FMAs: all threads, after the units.
+__device__ __noinline__ void sum_marked(const RedArgs &a) {
+  for (long long u = blockIdx.x; u < a.units; u += gridDim.x) {
+    const Unit w = unit_of(a, u);
+    const int nc = min(128, a.C - w.c0), nq = min(kDigN, a.r - w.q0);
+    double *out = a.out + w.blk * a.r * a.C + (long long)w.c0 * a.r + w.q0;
+    const double *V = a.V + w.row0 + (long long)w.q0 * a.ldv, *X = a.X + w.row0 + (long long)w.c0 * a.ldx;
+    for (int e = threadIdx.x; e < nc * nq; e += kThreads) {
+      const int q = e % nq, c = e / nq;
+      double *o = out + q + (long long)c * a.r;
+      if (!isnan(*o)) continue;
+      double s = 0.0;
+      for (int i = 0; i < w.rows; ++i) s = fma(V[i + q * a.ldv], X[i + c * a.ldx], s);
+      *o = s;
+    }
+  }
 }
 
 }  // namespace
@@ -106,7 +127,8 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
     const bool hit = wf.cta == (int)blockIdx.x;
     sh->skip = hit ? wf.stage : -1;
     sh->budget = hit && wf.budget > 0 ? wf.budget : kWait;
-    sh->abort = 0;
+    sh->abort = sh->marked = 0;
+    sh->args = a;
     mbar_fence_init();
   }
   for (int e = tid; e < 4 * kGroup; e += kThreads) sh->rowmax[0][e] = 0;
@@ -356,7 +378,10 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
         double *o = a.out + w.blk * a.r * a.C + (long long)(w.c0 + row) * a.r + w.q0 + 16 * h;
 #pragma unroll
         for (int c = 0; c < 16; ++c)
-          if (w.q0 + 16 * h + c < a.r) o[c] = acc[c];
+          if (w.q0 + 16 * h + c < a.r) {
+            o[c] = acc[c];
+            if (isnan(acc[c])) sh->marked = 1;
+          }
       }
     }
   }
@@ -368,6 +393,7 @@ __global__ void __launch_bounds__(kThreads, 1) f64_reduce_tc_kernel(RedArgs a) {
     tc_fence_after();
     tc_dealloc(tmem, 2 * kDigAccCols);
   }
+  if (sh->marked && !sh->abort) sum_marked(sh->args);
 }
 
 // Row chunks per block: of the counts that fill one, two, .. `per_sm` waves of

@@ -29,9 +29,11 @@
 // unknowns or equations in other units, which FP64 FMAs do not notice --
 // leaves the digits as they are.
 //
-// Non-finite operands: a group holding an infinity or NaN makes every result
-// it enters NaN (an FP64 FMA chain gives NaN or infinity there).  Subnormal
-// operands count as zero.
+// Non-finite operands: a group holding an infinity or NaN is marked.  The update and
+// the reduction go over the results it enters again at a CTA's end and form them by
+// FP64 FMAs (in the loops the calls would cost the update's epilogue 60 %).  The leaf
+// application, whose operand is overwritten by then, gives NaN; solves refuse such
+// right-hand sides.  Subnormal operands count as zero.
 #pragma once
 #include <cuda_fp16.h>
 
@@ -65,6 +67,12 @@ __device__ __forceinline__ void dig_key(int &key, unsigned h, int c) {  // h: hi
 }
 __device__ __forceinline__ int dig_scale(int key, unsigned ahi_max, int zero) {
   return ahi_max >= 0x7ff00000u ? kDigBad : key == kDigZero ? zero : key;
+}
+// The mark of a group, from memory: n values, `stride` apart.
+__device__ __forceinline__ bool dig_marked(const double *x, long long stride, int n) {
+  bool finite = true;
+  for (int k = 0; k < n; ++k) finite = finite && dig_ahi(x[k * stride]) < 0x7ff00000u;
+  return !finite;
 }
 constexpr int kDigZeroA = 0, kDigZeroB = 2046;  // scales of groups of zeros (any usual one: their sums are 0)
 
@@ -207,10 +215,10 @@ __device__ __forceinline__ long long dig_combine(const unsigned (&v)[kDiag][W], 
 // v 2^(t - 2099) rounded to FP64, t the sum of the two groups' scales: packed
 // on the integer pipes (the FP64 pipe's conversion takes three times as long
 // as its additions; with it the low-rank update took 7800 clocks a tile
-// instead of 5000).  Out of line: results outside the normal range,
-// non-finite operands.
-static __device__ __noinline__ double dig_value_any(long long v, int t) {
-  if (t >= kDigBad / 2) return __longlong_as_double(0x7ff8000000000000ll);
+// instead of 5000).  Out of line: results outside the normal range, and marked
+// groups.
+template <bool NAN_IF_MARKED = true> static __device__ __noinline__ double dig_value_any(long long v, int t) {
+  if (t >= kDigBad / 2) return NAN_IF_MARKED ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
   return scalbn((double)v, t - 2099);
 }
 // `odd` is set when the result has to come from dig_value_any instead.

@@ -45,6 +45,8 @@ struct Shared {
   long long budget;  // of the wait the hook lets run out, in SM clocks
   int skip;          // test hook: the stage whose digits are never announced (-1: none)
   unsigned tmem;
+  int marked;       // a group with an infinity or a NaN was met
+  UpdateArgs args;  // for add_marked (the address of a kernel's parameter costs registers)
   int abort;
 };
 
@@ -75,6 +77,42 @@ struct Walk {
   }
 };
 
+// The products of marked rows of A and columns of B, left out of a CTA's tiles
+// [t0, t1), added by FMAs: all threads, after the tiles.
+__device__ __noinline__ void add_marked(const UpdateArgs &a, int nrt, int nct, int t0, int t1, unsigned char *smem) {
+  double *sb = reinterpret_cast<double *>(smem);  // the tile's columns of op(B): [32][64]
+  bool *row = reinterpret_cast<bool *>(sb + kDigN * 64), *column = row + 128;
+  for (Walk w(nrt, nct, t0); w.t < t1; w.next()) {
+    const int j0 = w.ct * kDigN, nr = min(128, a.M - w.i0), nc = min(kDigN, a.N - j0);
+    const double *A = static_cast<const double *>(a.A) + (long long)w.b * a.a_bstride + w.i0;
+    const double *B = a.B + (long long)(w.b >> 1) * a.b_s1 + (long long)((w.b & 1) ^ a.b_flip) * a.b_s2;
+    double *C = static_cast<double *>(a.C) + (long long)w.b * a.c_bstride + w.i0 + (long long)j0 * a.ldc;
+    __syncthreads();
+    for (int e = threadIdx.x; e < nc * a.K; e += kThreads) {
+      const int j = j0 + e / a.K, q = e % a.K;
+      double v = a.b_trans ? B[j + (long long)q * a.ldb] : B[q + (long long)j * a.ldb];
+      if (a.scale) v *= a.scale_cols ? a.scale[j] : a.scale[q];
+      sb[e / a.K * 64 + q] = v;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nr + nc; e += kThreads) {
+      if (e < nr)
+        row[e] = dig_marked(A + e, a.lda, a.K);
+      else
+        column[e - nr] = dig_marked(sb + (e - nr) * 64, 1, a.K);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nr * nc; e += kThreads) {
+      const int i = e % nr, j = e / nr;
+      if (!row[i] && !column[j]) continue;
+      double s = 0.0;
+      for (int q = 0; q < a.K; ++q) s = fma(A[i + (long long)q * a.lda], sb[j * 64 + q], s);
+      double *c = C + i + (long long)j * a.ldc;
+      *c = fma(a.alpha, s, *c);
+    }
+  }
+}
+
 }  // namespace
 
 template <int KC>
@@ -102,7 +140,8 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
     const bool hit = wf.cta == (int)blockIdx.x;
     sh->skip = hit ? wf.stage : -1;
     sh->budget = hit && wf.budget > 0 ? wf.budget : kWait;
-    sh->abort = 0;
+    sh->abort = sh->marked = 0;
+    sh->args = a;
     mbar_fence_init();
   }
   if (warp == kMmaWarp) {
@@ -222,6 +261,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
         // were issued, two tiles after those of rt - 4 at least, once the epilogue had
         // freed that set -- and read the scales this slot held.
         if (half == 0) sh->ea[rt & 3][ht] = dig_scale(key, mx, kDigZeroA);
+        if (mx >= 0x7ff00000u) sh->marked = 1;
 #pragma unroll
         for (int c = 0; c < KC; ++c)
 #pragma unroll
@@ -272,6 +312,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
           mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, x));
         }
         if (o == 0) sh->eb[ti & 7][col] = dig_scale(key, mx, kDigZeroB);
+        if (mx >= 0x7ff00000u) sh->marked = 1;
         if (8 * o < 16 * ksteps)
           dig_put8(pb + (slot * KC + o / 4) * kDigBBytes, kDigBPlane, swz64(col, o & 3), xb[p],
                    [&](int e) { return bx[e]; }, key);
@@ -348,7 +389,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
 #pragma unroll
         for (int c = 0; c < 2; ++c) x[c] = dig_value(dig_combine<32 * KC>(v, c), ea + eb[c], odd);
         if (odd)
-          for (int c = 0; c < 2; ++c) x[c] = dig_value_any(dig_combine<32 * KC>(v, c), ea + eb[c]);
+          for (int c = 0; c < 2; ++c) x[c] = dig_value_any<false>(dig_combine<32 * KC>(v, c), ea + eb[c]);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const int cc = c2 + c;
@@ -368,6 +409,7 @@ f64_update_tc_kernel(UpdateArgs a, int nrt, int nct, int ntiles, DevStatus *st) 
     tc_fence_after();
     tc_dealloc(tmem, 2 * kDigAccCols);
   }
+  if (sh->marked && !sh->abort) add_marked(sh->args, nrt, nct, t0, t1, pa);
 }
 
 template <int KC>
