@@ -1782,12 +1782,17 @@ int hodlr_factor(hodlr_handle h) {
 }
 
 // Independent handles factored side by side, handle i's work on streams[i] after
-// what its own stream holds.  The first failure is returned, *bad its index; handles
-// after one whose work could not be enqueued are left as they are.
+// what its own stream holds.  The first failure is returned, *bad its index; the
+// handles after it are left factored only if they were (from the same inputs: setting
+// one unfactors its handle).
 namespace hodlr {
 int hodlr_factor_many(hodlr_handle *h, int count, const cudaStream_t *streams, cudaEvent_t fork, int *bad) {
   std::vector<cudaStream_t> own(count);
-  for (int i = 0; i < count; ++i) own[i] = h[i]->st;
+  std::vector<char> was(count);
+  for (int i = 0; i < count; ++i) {
+    own[i] = h[i]->st;
+    was[i] = h[i]->factored;
+  }
   int begun = 0, rc = HODLR_OK;
   for (; begun < count && rc == HODLR_OK; ++begun) {
     if (cudaEventRecord(fork, own[begun]) != cudaSuccess ||
@@ -1812,6 +1817,7 @@ int hodlr_factor_many(hodlr_handle *h, int count, const cudaStream_t *streams, c
     cudaStreamSynchronize(streams[i]);
     h[i]->st = own[i];
   }
+  for (int i = first + 1; i < begun; ++i) h[i]->factored = h[i]->factored && was[i];
   *bad = first;
   return rc == HODLR_OK ? rc : set_err(rc, why);
 }
