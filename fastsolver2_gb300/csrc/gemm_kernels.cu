@@ -442,13 +442,13 @@ static bool tensor_cores_off() {
 template <typename T, typename OutT>
 static cudaError_t reduce_dispatch(const T *A, long long lda, const T *X, long long ldx, long long nrows,
                                    int nbatch, int r, int C, OutT *out, double *work, const int *skip,
-                                   cudaStream_t s, DevStatus *st) {
+                                   cudaStream_t s, DevStatus *st, bool native) {
   int nchunks, chunk_rows;
   reduce_plan(nrows, nbatch, C, current_tuning().red_ctas_per_sm * kNumSMs, nchunks, chunk_rows);
   // FP64 on the tensor cores from 9 columns on, the widest the thin FMA tile
   // takes (up to 8): a 64-column FMA tile of 64 rows and 32 ranks takes 32 us of
   // an SM, a group of the tensor-core kernel (128 columns) 4
-  const bool f64_tc = sizeof(T) == 8 && C > 8 && !tensor_cores_off();
+  const bool f64_tc = sizeof(T) == 8 && C > 8 && !native && !tensor_cores_off();
   if (f64_tc) {
     int most, unused;  // the workspace's chunks
     reduce_plan(nrows, nbatch, C, kMaxRedCtasPerSm * kNumSMs, most, unused);
@@ -507,19 +507,19 @@ static cudaError_t reduce_dispatch(const T *A, long long lda, const T *X, long l
 template <typename T>
 cudaError_t launch_reduce_tn(const T *A, long long lda, const T *X, long long ldx, long long nrows,
                              int nbatch, int r, int C, double *out, double *work, const int *skip,
-                             cudaStream_t s, DevStatus *st, float *out32) {
+                             cudaStream_t s, DevStatus *st, float *out32, bool native) {
   if (C <= 0 || nbatch <= 0) return cudaSuccess;
   if (r < 1 || r > 64) return cudaErrorInvalidValue;
-  if (out32) return reduce_dispatch<T, float>(A, lda, X, ldx, nrows, nbatch, r, C, out32, work, skip, s, st);
-  return reduce_dispatch<T, double>(A, lda, X, ldx, nrows, nbatch, r, C, out, work, skip, s, st);
+  if (out32) return reduce_dispatch<T, float>(A, lda, X, ldx, nrows, nbatch, r, C, out32, work, skip, s, st, native);
+  return reduce_dispatch<T, double>(A, lda, X, ldx, nrows, nbatch, r, C, out, work, skip, s, st, native);
 }
 
 template cudaError_t launch_reduce_tn<double>(const double *, long long, const double *, long long, long long,
                                               int, int, int, double *, double *, const int *, cudaStream_t,
-                                              DevStatus *, float *);
+                                              DevStatus *, float *, bool);
 template cudaError_t launch_reduce_tn<float>(const float *, long long, const float *, long long, long long, int,
                                              int, int, double *, double *, const int *, cudaStream_t, DevStatus *,
-                                             float *);
+                                             float *, bool);
 
 // ------------------------------------------------------------------ K5
 // CTA tile 128 rows x 64 columns, K staged 32 at a time; each thread owns
@@ -785,7 +785,7 @@ cudaError_t launch_update_nn(const UpdateArgs &a, cudaStream_t s, DevStatus *st)
     // SM on the tensor cores, and 8 columns 8 us on the FMA pipe (rank 32)
     if (!a.a_trans && a.K <= 4) return launch_f64_thin_outer(a, s);
     if (!a.a_trans && a.N <= 4 && !a.overwrite) return launch_f64_thin_update(a, s);
-    if (!tensor_cores_off() && f64_update_tc_try(a, st, s, e)) return e;
+    if (!a.native && !tensor_cores_off() && f64_update_tc_try(a, st, s, e)) return e;
     if (a.overwrite) return cudaErrorInvalidValue;  // the others add to C
     if (!a.a_trans && a.N <= 8) return launch_f64_thin_update(a, s);
   }

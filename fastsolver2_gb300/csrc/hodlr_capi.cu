@@ -768,9 +768,11 @@ static int solve_sweep(hodlr_ctx *h, T *X, long long ldx, int k, bool trans, con
   return HODLR_OK;
 }
 
-// Y = beta*Y0 + alpha * op(A) X in native FP64 (Y0 == nullptr: Y starts at 0).
+// Y = beta*Y0 + alpha * op(A) X in FP64 (Y0 == nullptr: Y starts at 0); native: by
+// FMAs only, for callers who chose that arithmetic (HODLR_RESID_FP64).
 static int matvec_fp64(hodlr_ctx *h, bool trans, const double *X, long long ldx, const double *Y0,
-                       long long ldy0, double *Y, long long ldy, int k, double alpha, const int *skip) {
+                       long long ldy0, double *Y, long long ldy, int k, double alpha, const int *skip,
+                       bool native = false) {
   const long long n = h->n;
   const int m = h->m, L = h->L, r = h->r;
   cudaStream_t s = h->st;
@@ -796,6 +798,7 @@ static int matvec_fp64(hodlr_ctx *h, bool trans, const double *X, long long ldx,
   la.nbatch = h->nleaf;
   la.alpha = alpha;
   la.skip = skip;
+  la.native = native;
   PHASE(h, HODLR_PHASE_RESID_LEAF, launch_update_nn<double>(la, s, h->dst));
   for (int l = 0; l < L; ++l) {
     const int nb = h->nb(l);
@@ -803,7 +806,7 @@ static int matvec_fp64(hodlr_ctx *h, bool trans, const double *X, long long ldx,
     const double *Ared = trans ? h->Ulev(l) : h->Vlev(l);
     const double *Aupd = trans ? h->Vlev(l) : h->Ulev(l);
     PHASE(h, HODLR_PHASE_RESID_REDUCE,
-          launch_reduce_tn<double>(Ared, n, X, ldx, rows, nb, r, k, h->Tbuf, h->red, skip, s, h->dst));
+          launch_reduce_tn<double>(Ared, n, X, ldx, rows, nb, r, k, h->Tbuf, h->red, skip, s, h->dst, nullptr, native));
     UpdateArgs ua{};
     ua.A = Aupd;
     ua.lda = n;
@@ -823,6 +826,7 @@ static int matvec_fp64(hodlr_ctx *h, bool trans, const double *X, long long ldx,
     ua.nbatch = nb;
     ua.alpha = alpha;
     ua.skip = skip;
+    ua.native = native;
     PHASE(h, HODLR_PHASE_RESID_UPDATE, launch_update_nn<double>(ua, s, h->dst));
   }
   return HODLR_OK;
@@ -939,7 +943,7 @@ static int residual(hodlr_ctx *h, bool trans, const double *X, long long ldx, co
                     double *R, long long ldr, int k, const int *skip) {
   if (h->oz && !trans) return residual_tensor(h, const_cast<double *>(X), ldx, B, ldb, R, ldr, k, skip);
   if (h->emulated) return residual_emulated(h, trans, X, ldx, B, ldb, R, ldr, k, skip);
-  return matvec_fp64(h, trans, X, ldx, B, ldb, R, ldr, k, -1.0, skip);
+  return matvec_fp64(h, trans, X, ldx, B, ldb, R, ldr, k, -1.0, skip, true);
 }
 
 // While the handle's stream is being captured (and no per-phase event nodes

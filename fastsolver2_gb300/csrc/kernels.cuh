@@ -128,7 +128,7 @@ cudaError_t f64_leaf_tc_set_wait_fault(const WaitFault &wf);
 template <typename T>
 cudaError_t launch_reduce_tn(const T *A, long long lda, const T *X, long long ldx, long long nrows,
                              int nbatch, int r, int C, double *out, double *work, const int *skip,
-                             cudaStream_t s, DevStatus *st = nullptr, float *out32 = nullptr);
+                             cudaStream_t s, DevStatus *st = nullptr, float *out32 = nullptr, bool native = false);
 
 // K5: C_b += alpha * A_b * diag(scale) * op(B_b) for b in [0, nbatch):
 //   A_b = A + b*a_bstride (M x K, lda), C_b = C + b*c_bstride (M x N, ldc),
@@ -148,6 +148,7 @@ struct UpdateArgs {
   // C_b = instead of += (its old values are not read): FP64 with K <= 4, or on
   // the tensor cores
   int overwrite;
+  int native;  // FP64: by FMAs, whatever the shape
 };
 // f64_thin.cu: the FP64 steps for up to 8 columns (update, reduction, leaf and
 // capacitance application), and updates of an inner dimension up to 4
