@@ -21,9 +21,10 @@ template <typename T> __device__ __forceinline__ void swap_vals(T &a, T &b) {
   b = t;
 }
 
-// 1 / x to FP64 accuracy for |x| in 2^-960 .. 2^960 (rcp_usual): the third-order
-// iteration y <- y (1 + e + e^2), e = 1 - x y, on the hardware's approximation,
-// which triples its correct bits (20); three FMAs where a division takes 440 clocks.
+// 1 / x within 0.52 ulp for |x| in 2^-960 .. 2^961 (rcp_usual): the hyperpower
+// iteration of order three (Altman, Pacific J. Math. 10, 1960), y <- y (1 + e + e^2)
+// with e = 1 - x y, on the hardware's approximation.  Its 20 correct bits become 60:
+// 2^-7 ulp, and the last FMA rounds once.  Three FMAs where a division takes 440 clocks.
 __device__ __forceinline__ double newton_rcp(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -33,6 +34,29 @@ __device__ __forceinline__ double newton_rcp(double x) {
 __device__ __forceinline__ bool rcp_usual(double x) {
   return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 63u < 1921u;
 }
+
+// Quotients by one divisor, in FP64 by its reciprocal in two parts, hi + lo = 1 / u to
+// 2^-104: x hi + x lo with one rounding of the sum, so within 0.5 + 2^-40 ulp of x / u
+// and another value than the division's only that close to the middle of two; within
+// an ulp where the quotient or its second part is subnormal.  Extreme divisors,
+// infinities and NaNs are left to the division.
+template <typename T> struct Quotient {
+  T u;
+  __device__ __forceinline__ static Quotient by(T u) { return Quotient{u}; }
+  __device__ __forceinline__ T of(T x) const { return x / u; }
+};
+template <> struct Quotient<double> {
+  double u, hi, lo;
+  int ok;
+  __device__ __forceinline__ static Quotient by(double u) {
+    const double hi = 1.0 / u;
+    return Quotient{u, hi, fma(-u, hi, 1.0) * hi, fabs(u) > 1e-280 && fabs(u) < 1e280};
+  }
+  __device__ __forceinline__ double of(double x) const {  // x / u
+    const double q = fma(x, hi, x * lo);
+    return ok && isfinite(q) ? q : x / u;
+  }
+};
 
 // In-place LU with partial pivoting of the m x m matrix A (lda).  piv gets the
 // 1-based LAPACK pivots.  *info = 0, or k+1 for the first zero pivot k.  The

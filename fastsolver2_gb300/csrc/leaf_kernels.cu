@@ -122,26 +122,6 @@ leaf_getrs_kernel(const T *__restrict__ LU, const int *__restrict__ ipiv, int m,
   }
 }
 
-// Quotients by one divisor, in FP64 by its reciprocal in two parts: rounded as the
-// division rounds but for extreme exponents, which are left to it.
-template <typename T> struct Quotient {
-  T u;
-  __device__ __forceinline__ static Quotient by(T u) { return Quotient{u}; }
-  __device__ __forceinline__ T of(T x) const { return x / u; }
-};
-template <> struct Quotient<double> {
-  double u, hi, lo;
-  int ok;
-  __device__ __forceinline__ static Quotient by(double u) {
-    const double hi = 1.0 / u;
-    return Quotient{u, hi, fma(-u, hi, 1.0) * hi, fabs(u) > 1e-280 && fabs(u) < 1e280};
-  }
-  __device__ __forceinline__ double of(double x) const {  // x / u
-    const double q = fma(x, hi, x * lo);
-    return ok && isfinite(q) ? q : x / u;
-  }
-};
-
 // X := D^{-1} X for many columns: 32-row diagonal blocks in launches of their own --
 // 32 columns a CTA, lane = column, each of the four warps with every fourth row in
 // registers, row k passed through shared memory once it is done, a step a barrier
