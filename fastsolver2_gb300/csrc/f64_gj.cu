@@ -1,26 +1,35 @@
 // K1 in FP64 for leaves of 64, 128 and 256 rows whose factorisation only needs
 // the explicit inverse, and K4a in FP64, the capacitance systems' LU and
-// inverse: blocked Gauss-Jordan with partial pivoting, 32 columns a block, the
-// O(m^3) part on the tensor cores.
+// inverse: elimination with partial pivoting, 32 columns a block, the O(m^3) part
+// on the tensor cores.
 //
-// For the pivot rows K and columns K of a block (D = A_KK after the block's row
-// interchanges, L11 U11 = D its LU), every other row I and column J:
-//     A_KJ <- D^-1 A_KJ      A_IJ <- A_IJ - (A_IK D^-1) A_KJ
-//     A_KK <- D^-1           A_IK <- -A_IK D^-1
+// Up to 128 rows in one phase, Gauss-Jordan.  For the pivot rows K and columns K of a
+// block (after the block's row interchanges A_KK = L11 U11), every other row I, W_I =
+// A_IK U11^-1 (below the block the multipliers of the LU), W_K = -U11^-1, and all
+// columns J, those of K begun anew as the identity's:
+//     R_J = L11^-1 A_KJ      A_IJ <- A_IJ - W_I R_J      A_KJ <- -W_K R_J
+// Leaves of 256 rows in two phases, the LU with L^-1 beside it (rows I below only, A_KJ
+// <- R_J), then U^-1 times L^-1 from the last block up (R = U11^-1 Z_K, Z_I <- Z_I -
+// U_IK R above).
+//
 // The panel kernel (one CTA a leaf, one thread a row) factors the block's
 // columns with the pivot rule of dgetf2 (first row of largest |a| among the
-// rows not pivoted yet, reciprocal scaling), forms W = A_IK D^-1 as (A_IK
-// U11^-1) L11^-1 -- for the rows below, the multipliers of the LU times L11^-1,
-// so that no product is larger than elimination makes it -- interchanges the
-// rows of the other columns, moves the pivot rows out into R and leaves zeros
-// in their place; then one batched product A <- A - W R over all leaves
-// (f64_update_tc.cu, W's pivot rows -D^-1) does both updates.  The LU factors
-// and pivots of these leaves are formed on request from the blocks themselves
-// (leaf_factor_reg_kernel / leaf_blocked.cu); those of a capacitance system
-// (padded with the identity to 32, 64 or 128 rows), and of leaves whose caller
-// wants them in any case, are captured as they appear:
-// L11, U11 and L21 in the panel, U12 = L11^-1 A_KJ from R by warps that have no
-// rows, later interchanges applied to the columns of L already out.
+// rows not pivoted yet, reciprocal scaling), interchanges the rows of the other
+// columns, moves the pivot rows out into R and forms W and R; batched products over
+// all leaves (f64_update_tc.cu) do the updates.  The LU factors and pivots of these
+// leaves are formed on request from the blocks themselves (leaf_factor_reg_kernel /
+// leaf_blocked.cu); those of a capacitance system (padded with the identity to 32, 64
+// or 128 rows), and of leaves whose caller wants them in any case, are captured as they
+// appear: L11, U11 and L21 in the panel, U12 = R right of the block, later interchanges
+// applied to the columns of L already out.
+//
+// Backward error.  The sums are those of the sweeps before, entry by entry (reg_factor.cuh:
+// Gauss-Jordan; leaf_blocked.cu: substitution on the identity), so that A x = b and
+// A^T x = b keep their residuals.  Two orders that cost less do not: W_I L11^-1 in place
+// of R makes the residual of A x = b grow with the condition (1e6: 60 times, 1e10 4000
+// times, leaves of 64 rows), and one product for the rows above and in the block, whose
+// W are as large as 1 / U11's pivots, and for those below, whose W are at most 1, that of
+// A^T x = b: the digits of a row tile share the balance of an inner index.
 //
 // A leaf or system with a pivot below 2^-40 of the largest entry of its row and of its
 // column of D -- singular, or so close to it that the two ways of rounding
@@ -28,16 +37,16 @@
 // (leaf_gj_again_kernel, cap_factor_kernel), which decides on a zero pivot and
 // gives its inverse.
 //
-// What bounds it: the FP64 pipe, by the panels: (m + 32) (32^2 - 32) FMAs each,
-// 0.6 M for leaf 128 of the 2.1 M of its Gauss-Jordan sweep in one piece.  32
+// What bounds it: the FP64 pipe, by the panels: some (2 m + 32) 496 FMAs each in one
+// phase, 0.57 M for leaf 128 of the 2.1 M of its Gauss-Jordan sweep in one piece.  32
 // columns a block: at 16 the panels would take half as long, but each of twice
 // as many products reads and writes the whole matrix.  Measured with the digit
-// images: 8192 leaves of 128 rows 13.6 ms, 69.7 by the register-resident sweep
+// images: 8192 leaves of 128 rows 15.4 ms, 69.7 by the register-resident sweep
 // (leaf_factor_reg_kernel, at 39 % of the FP64 rate); 16 leaves of 256 rows 1.34
 // ms, 2.50 by blocked LU and triangular solves.  The capacitance systems of N =
-// 2^20, rank 32 (8191 of 64 rows in 13 levels): 6 ms with their applications to
-// the transformed bases on the tensor cores 9, 38 by the register-resident sweep
-// (cap_factor_reg_kernel) and FMA applications; a lone system 230 us, 308 before.
+// 2^20, rank 32 (8191 of 64 rows in 13 levels) with their applications to the transformed
+// bases on the tensor cores 11.4 ms, 38 by the register-resident sweep
+// (cap_factor_reg_kernel) and FMA applications; a lone system of 64 rows 190 us.
 #include <algorithm>
 
 #include "dense_ops.cuh"
@@ -50,6 +59,7 @@ cudaError_t launch_cap_factor_marked(const CapFactorArgs &a, const int *only, cu
 
 namespace {
 constexpr int kNb = 32;
+template <int M> constexpr bool kGjTwo = M == 256;  // see above
 
 // Where a panel puts the LU factors (capacitance systems): n x n of the M x M
 // padded system, DGETRF's layout, 1-based pivots.
@@ -63,20 +73,21 @@ struct LuOut {
 // is worked on in place; W [block][32][m] (column c at + c m), R [block][m][32]
 // (column j at + 32 j), perm [block][m]: the original row at each position.
 //
-// One thread a row, the panel's 32 columns in its registers; the identity's rows
-// go along and become U11^-1, then D^-1.  An FP64 FMA holds its sub-partition's
+// One thread a row, the panel's 32 columns in its registers; in one phase the
+// identity's rows go along and become U11^-1.  An FP64 FMA holds its sub-partition's
 // pipe for 64 clocks (and its result comes then), so a step is 64 clocks for
 // each column left, plus some 900 for the pivot: one block barrier, every warp
 // finding its best candidate for the next pivot as soon as that column is up to
 // date, computing its reciprocal beside the other columns' FMAs, and leaving the
 // whole row in shared memory, so that after the barrier every thread reads the
-// winner's.  A lone 64-row panel takes 66 us (74000 clocks the elimination, 32000
-// the product with L11^-1); with two barriers, a division after the first and
-// FP64 compares it took 87 to 108.
-template <int M, bool LU> __host__ __device__ constexpr int gj_threads() { return LU ? 2 * M : M + kNb; }
+// winner's.  Then the threads take a column each of L11^-1 A_KJ.  A lone 64-row panel
+// takes 66 us (74000 clocks the elimination, 32000 the columns); with two barriers, a
+// division after the first and FP64 compares it took 87 to 108.
+template <int M> __host__ __device__ constexpr int gj_threads() { return kGjTwo<M> ? M : M + kNb; }
 template <int M, bool LU>
-__global__ void __launch_bounds__(gj_threads<M, LU>())
+__global__ void __launch_bounds__(gj_threads<M>(), M == 128 ? (LU ? 3 : 4) : M == 64 ? 5 : 0)
 gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, int nc, const unsigned *big, int *again, LuOut out) {
+  constexpr bool kTwo = kGjTwo<M>, kOne = M == kNb;  // two phases; a single block
   constexpr int NW = M / 32;  // warps with rows of the block; the next has the identity's
   __shared__ double sU[2][NW][kNb], sRcp[2][NW], sL[kNb][kNb];
   __shared__ uint4 sBest[2][NW];  // |a| (high, low word), position, row of each warp's candidate
@@ -151,7 +162,7 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, int nc, cons
       pos = (int)best.z;
     }
     if (LU && tid == 0 && k0 + c < out.n) out.ipiv[blk * out.n + k0 + c] = (int)best.z + 1;
-    const bool row = !pivot_row && (real || ident);  // pivot rows keep L11 and U11
+    const bool row = kTwo ? open : !pivot_row && (real || ident);  // pivot rows keep L11 and U11
     const double *u = sU[buf][bw];
     double l = 0.0;
     if (row) {
@@ -182,15 +193,42 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, int nc, cons
     for (int c = 0; c < kNb; ++c)
       if (k0 + c < out.n) lu[pos + (long long)(k0 + c) * out.n] = a[c];
   }
+  if (kOne) {  // D^-1 at once: the identity's rows times L11^-1 from the right
+    __syncthreads();
+    if (ident) {
+#pragma unroll
+      for (int t = kNb - 1; t > 0; --t) {
+        if (t >= nc) continue;
+#pragma unroll
+        for (int c = 0; c < t; ++c) a[c] -= a[t] * sL[t][c];
+      }
+#pragma unroll
+      for (int c = 0; c < kNb; ++c) Al[lane + (long long)c * M] = a[c];
+    }
+    if (real) perm[blk * M + pos] = orig;
+    return;
+  }
+  // W: the multipliers of the rows, and -U11^-1 in one phase.  The block's own columns
+  // begin anew, as those of the identity.
+  double *Wl = W + blk * M * kNb;
+  if (kTwo ? open : !pivot_row) {
+    const int row = real ? pos : k0 + lane;
+#pragma unroll
+    for (int c = 0; c < kNb; ++c) Wl[row + (long long)c * M] = real ? a[c] : -a[c];
+  }
+  if (kTwo ? real && tid >= k0 + kNb : real) {
+#pragma unroll
+    for (int c = 0; c < kNb; ++c) Al[tid + (long long)(k0 + c) * M] = 0.0;
+  }
   // the other columns: rows to their positions, the pivot rows into R, zeros in
   // their place; in the columns of L already out, the rows alone
   double *Rl = R + blk * M * kNb;
   const bool moves = real && (pos != tid || pivot_row);
   for (int j0 = 0; j0 < M; j0 += 8) {
+    if (j0 >= k0 && j0 < k0 + kNb) continue;
     double x[8], y[8];
-    const bool panel = j0 >= k0 && j0 < k0 + kNb;
     const bool moves_l = LU && j0 < k0 && real && tid >= k0 && tid < out.n && pos != tid;
-    if (moves && !panel)
+    if (moves)
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[e] = Al[tid + (long long)(j0 + e) * M];
     if (moves_l)
@@ -200,50 +238,81 @@ gj_panel_kernel(double *A, double *W, double *R, int *perm, int k0, int nc, cons
     if (moves_l && pos < out.n)
 #pragma unroll
       for (int e = 0; e < 8; ++e) lu[pos + (long long)(j0 + e) * out.n] = y[e];
-    if (moves && !panel)
+    if (moves && !(kTwo && pivot_row))
 #pragma unroll
       for (int e = 0; e < 8; ++e) Al[pos + (long long)(j0 + e) * M] = pivot_row ? 0.0 : x[e];
     if (pivot_row)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) Rl[(long long)(j0 + e) * kNb + pos - k0] = panel ? 0.0 : x[e];
+      for (int e = 0; e < 8; ++e) Rl[(long long)(j0 + e) * kNb + pos - k0] = x[e];
   }
   __syncthreads();
-  if (real) perm[blk * M + pos] = orig;
-  if (LU && warp > NW) {  // U12's column j, one a thread
-    const int j = k0 + kNb + tid - (M + kNb);
-    if (j < out.n) {
-      const double *Rj = Rl + (long long)j * kNb;
+  if (!real) return;
+  perm[blk * M + pos] = orig;
+  // column tid of L11^-1 [A_KJ, I]; U12 and, in two phases, what the pivot rows hold from now on
+  double *Rj = Rl + (long long)tid * kNb;
+  const int jk = tid - k0;  // of the block's own columns, from 0 on
+  const bool own = jk >= 0 && jk < kNb;
 #pragma unroll
-      for (int c = 0; c < kNb; ++c) a[c] = Rj[c];
+  for (int c = 0; c < kNb; ++c) a[c] = own ? (c == jk ? 1.0 : 0.0) : Rj[c];
 #pragma unroll
-      for (int c = 0; c < kNb; ++c) {
-        if (c >= nc) continue;
+  for (int c = 0; c < kNb; ++c) {
+    if (LU && c >= nc) continue;
 #pragma unroll
-        for (int t = c + 1; t < kNb; ++t) a[t] -= sL[t][c] * a[c];
-      }
-#pragma unroll
-      for (int c = 0; c < kNb; ++c)
-        if (k0 + c < out.n) lu[k0 + c + (long long)j * out.n] = a[c];
-    }
+    for (int t = c + 1; t < kNb; ++t) a[t] -= sL[t][c] * a[c];
   }
-  if (!pivot_row && (real || ident)) {
-    // times L11^-1 from the right: W, and the panel's new columns (the identity's
-    // rows, now D^-1, are the pivot rows')
 #pragma unroll
-    for (int t = kNb - 1; t > 0; --t) {
-      if (LU && t >= nc) continue;
+  for (int c = 0; c < kNb; ++c) Rj[c] = a[c];
+  if (LU && jk >= kNb && tid < out.n)
 #pragma unroll
-      for (int c = 0; c < t; ++c) a[c] -= a[t] * sL[t][c];
-    }
-    double *Wl = W + blk * M * kNb;
-    const int row = real ? pos : k0 + lane;
+    for (int c = 0; c < kNb; ++c)
+      if (k0 + c < out.n) lu[k0 + c + (long long)tid * out.n] = a[c];
+  if (kTwo) {
 #pragma unroll
-    for (int c = 0; c < kNb; ++c) {
-      const double v = real ? a[c] : -a[c];
-      Wl[row + (long long)c * M] = v;
-      Al[row + (long long)(k0 + c) * M] = -v;
-    }
+    for (int c = 0; c < kNb; ++c) Al[k0 + c + (long long)tid * M] = own && c <= jk ? sL[c][jk] : a[c];
   }
+}
+
+// Two phases, the columns of Z, at their places in D^-1, from L^-1 (below the diagonal of A).
+__global__ void __launch_bounds__(256) gj_split_kernel(const double *__restrict__ A, const int *__restrict__ perm, int m,
+                                                       double *Z) {
+  const long long leaf = blockIdx.x;
+  const double *Al = A + leaf * m * m;
+  double *Zl = Z + leaf * m * m;
+  for (int e = threadIdx.x; e < m * m; e += 256) {
+    const int i = e % m, p = e / m;
+    Zl[i + (long long)perm[leaf * m + p] * m] = i > p ? Al[e] : i == p ? 1.0 : 0.0;
+  }
+}
+
+// Rows K of Z times U11^-1 from the left, also into R: 32 columns a CTA (blockIdx.y),
+// four neighbouring lanes a column, every fourth row each (one thread a column takes
+// 32000 clocks, a leaf's 256 columns in one CTA 90000).
+__global__ void __launch_bounds__(4 * kNb) gj_rows_kernel(const double *__restrict__ A, int m, double *Z, double *R, int k0) {
+  constexpr int NC = kNb / 4;
+  __shared__ double sU[kNb][kNb + 1], sRcp[kNb];
+  const int tid = threadIdx.x, q = tid & 3, j = kNb * (int)blockIdx.y + (tid >> 2);
+  const long long blk = blockIdx.x;
+  const double *Akk = A + blk * m * m + (long long)k0 * (m + 1);
+  double *z = Z + blk * m * m + k0 + (long long)j * m, *Rj = R + (blk * m + j) * kNb;
+  for (int e = tid; e < kNb * kNb; e += 4 * kNb) sU[e % kNb][e / kNb] = Akk[e % kNb + (long long)(e / kNb) * m];
+  double a[NC];
+#pragma unroll
+  for (int t = 0; t < NC; ++t) a[t] = z[4 * t + q];
+  __syncthreads();
+  if (tid < kNb) sRcp[tid] = rcp_usual(sU[tid][tid]) ? 1.0 / sU[tid][tid] : 0.0;
+  __syncthreads();
+#pragma unroll
+  for (int c = kNb - 1; c >= 0; --c) {
+    double w = a[c / 4];  // of the lane whose row it is
+    w = sRcp[c] != 0.0 ? w * sRcp[c] : w / sU[c][c];
+    w = __shfl_sync(0xffffffffu, w, c & 3, 4);
+    if (q == (c & 3)) a[c / 4] = w;
+    if (q < (c & 3)) a[c / 4] -= w * sU[c / 4 * 4 + q][c];
+#pragma unroll
+    for (int t = 0; t < c / 4; ++t) a[t] -= w * sU[4 * t + q][c];
+  }
+#pragma unroll
+  for (int t = 0; t < NC; ++t) z[4 * t + q] = Rj[4 * t + q] = a[t];
 }
 
 // A = D, the largest |D| of every row and column (high words), again = 0; the
@@ -321,14 +390,38 @@ __global__ void __launch_bounds__(256) leaf_gj_columns_kernel(const double *__re
   }
 }
 
-// `count` m x m systems (m 64, 128 and 256, or 32, 64 and 128 with the LU
+// C[system](rows r0 .. r0 + rows) -= F[system](those rows, 32 columns) R[system].
+static cudaError_t gj_product(int m, int count, const double *F, long long f_stride, const double *R, double *C, int r0,
+                              int rows, DevStatus *st, cudaStream_t s) {
+  if (rows <= 0) return cudaSuccess;
+  UpdateArgs ua{};
+  ua.A = F + r0;
+  ua.lda = m;
+  ua.a_bstride = f_stride;
+  ua.B = R;
+  ua.ldb = kNb;
+  ua.b_s1 = 2LL * m * kNb;
+  ua.b_s2 = (long long)m * kNb;
+  ua.C = C + r0;
+  ua.ldc = m;
+  ua.c_bstride = (long long)m * m;
+  ua.M = rows;
+  ua.N = m;
+  ua.K = kNb;
+  ua.nbatch = count;
+  ua.alpha = -1.0;
+  cudaError_t e = cudaSuccess;
+  return f64_update_tc_try(ua, st, s, e) ? e : cudaErrorInvalidValue;
+}
+
+// One phase: `count` m x m systems (m 64 and 128, or 32, 64 and 128 with the LU
 // factors), worked on in place in A: on return A holds the inverses of the
 // interchanged rows.  Rows and columns from n on are the identity's.
 template <bool LU>
-static cudaError_t gj_blocks(int m, int n, int count, double *A, double *W, double *R, int *perm, const unsigned *big,
-                             int *again, const LuOut &out, DevStatus *st, cudaStream_t s) {
+static cudaError_t gj_one(int m, int n, int count, double *A, double *W, double *R, int *perm, const unsigned *big,
+                          int *again, const LuOut &out, DevStatus *st, cudaStream_t s) {
 #define HODLR_GJ(MV)                                                                                            \
-  HODLR_LAUNCH((gj_panel_kernel<MV, LU>), count, (gj_threads<MV, LU>()), 0, s, A, W, R, perm, k0, std::min(kNb, n - k0), big, again, \
+  HODLR_LAUNCH((gj_panel_kernel<MV, LU>), count, gj_threads<MV>(), 0, s, A, W, R, perm, k0, std::min(kNb, n - k0), big, again, \
                out)
   for (int k0 = 0; k0 < n; k0 += kNb) {
     if (m == 64) {
@@ -336,32 +429,33 @@ static cudaError_t gj_blocks(int m, int n, int count, double *A, double *W, doub
     } else if (m == 128) {
       HODLR_GJ(128);
     } else {
-      constexpr int MV = LU ? 32 : 256;
-      if (m != MV) return cudaErrorInvalidValue;
-      HODLR_GJ(MV);
+      if (!LU || m != kNb) return cudaErrorInvalidValue;
+      if constexpr (LU) HODLR_GJ(kNb);
+      break;  // no other columns
     }
-    if (m == kNb) break;  // no other columns
-    UpdateArgs ua{};
-    ua.A = W;
-    ua.lda = m;
-    ua.a_bstride = (long long)m * kNb;
-    ua.B = R;
-    ua.ldb = kNb;
-    ua.b_s1 = 2LL * m * kNb;
-    ua.b_s2 = (long long)m * kNb;
-    ua.C = A;
-    ua.ldc = m;
-    ua.c_bstride = (long long)m * m;
-    ua.M = m;
-    ua.N = m;
-    ua.K = kNb;
-    ua.nbatch = count;
-    ua.alpha = -1.0;
-    cudaError_t e = cudaSuccess;
-    if (!f64_update_tc_try(ua, st, s, e)) return cudaErrorInvalidValue;
+    cudaError_t e = gj_product(m, count, W, (long long)m * kNb, R, A, 0, k0 + kNb, st, s);
+    if (e == cudaSuccess) e = gj_product(m, count, W, (long long)m * kNb, R, A, k0 + kNb, m - k0 - kNb, st, s);
     if (e != cudaSuccess) return e;
   }
 #undef HODLR_GJ
+  return cudaGetLastError();
+}
+
+// Two phases, leaves of 256 rows: Z = their inverses; A is worked on in place.
+static cudaError_t gj_two(int count, double *A, double *Z, double *W, double *R, int *perm, const unsigned *big,
+                          int *again, DevStatus *st, cudaStream_t s) {
+  constexpr int M = 256;
+  cudaError_t e;
+  for (int k0 = 0; k0 < M; k0 += kNb) {
+    HODLR_LAUNCH((gj_panel_kernel<M, false>), count, gj_threads<M>(), 0, s, A, W, R, perm, k0, kNb, big, again,
+                 (LuOut{nullptr, nullptr, 0}));
+    if ((e = gj_product(M, count, W, (long long)M * kNb, R, A, k0 + kNb, M - k0 - kNb, st, s)) != cudaSuccess) return e;
+  }
+  HODLR_LAUNCH(gj_split_kernel, count, 256, 0, s, A, perm, M, Z);
+  for (int k0 = M - kNb; k0 >= 0; k0 -= kNb) {
+    HODLR_LAUNCH(gj_rows_kernel, dim3(count, M / kNb), 4 * kNb, 0, s, A, M, Z, R, k0);
+    if ((e = gj_product(M, count, A + (long long)k0 * M, (long long)M * M, R, Z, 0, k0, st, s)) != cudaSuccess) return e;
+  }
   return cudaGetLastError();
 }
 
@@ -380,10 +474,11 @@ cudaError_t launch_f64_leaf_gj(const double *D, long long d_ld, long long d_stri
   unsigned *big = reinterpret_cast<unsigned *>(perm + (size_t)nleaf * m);
   int *again = reinterpret_cast<int *>(big + (size_t)nleaf * 2 * m);
   HODLR_LAUNCH(leaf_gj_copy_kernel, nleaf, 256, 0, s, D, d_ld, d_stride, m, A, big, again, st);
-  cudaError_t e = LU ? gj_blocks<true>(m, m, nleaf, A, W, R, perm, big, again, LuOut{LU, ipiv, m}, st, s)
-                     : gj_blocks<false>(m, m, nleaf, A, W, R, perm, big, again, LuOut{nullptr, nullptr, 0}, st, s);
+  cudaError_t e = m == 256 ? gj_two(nleaf, A, Dinv, W, R, perm, big, again, st, s)
+                  : LU     ? gj_one<true>(m, m, nleaf, A, W, R, perm, big, again, LuOut{LU, ipiv, m}, st, s)
+                           : gj_one<false>(m, m, nleaf, A, W, R, perm, big, again, LuOut{nullptr, nullptr, 0}, st, s);
   if (e != cudaSuccess) return e;
-  HODLR_LAUNCH(leaf_gj_columns_kernel, nleaf, 256, 0, s, A, perm, m, Dinv);
+  if (m != 256) HODLR_LAUNCH(leaf_gj_columns_kernel, nleaf, 256, 0, s, A, perm, m, Dinv);
   HODLR_LAUNCH(leaf_gj_again_kernel, nleaf, 256, 0, s, D, d_ld, d_stride, m, LU ? LU : A, ipiv, Dinv, again, st);
   return cudaGetLastError();
 }
@@ -453,7 +548,7 @@ cudaError_t launch_f64_cap_gj(const CapFactorArgs &a, void *scratch, cudaStream_
   int *again = reinterpret_cast<int *>(big + nn * 2 * m);
   const LuOut out{a.cap_lu + (long long)a.node_base * n2 * n2, a.cap_ipiv + (long long)a.node_base * n2, n2};
   HODLR_LAUNCH(cap_gj_build_kernel, a.nnode, 256, 0, s, a, m, A, big, again);
-  cudaError_t e = gj_blocks<true>(m, n2, a.nnode, A, W, R, perm, big, again, out, a.st, s);
+  cudaError_t e = gj_one<true>(m, n2, a.nnode, A, W, R, perm, big, again, out, a.st, s);
   if (e != cudaSuccess) return e;
   const long long base = (long long)a.node_base * n2 * n2;
   HODLR_LAUNCH(cap_gj_columns_kernel, a.nnode, 256, 0, s, A, perm, m, n2, a.sinv ? a.sinv + base : nullptr,
