@@ -811,7 +811,7 @@ def run_ragged(args, fs, torch, stream, colmajor):
         out[name]["max_rel_residual"] = worst
     del solutions
     out["residual_note"] = ("max over systems and columns of ||b - A x|| / ||b||, A x by each system's own FP64 "
-                            "handle (hodlr_matvec, native FP64)")
+                            "handle (hodlr_matvec, FP64)")
     for rep in range(2):   # the first pass loads and captures, the second is timed
         torch.cuda.synchronize()
         t0 = time.perf_counter()

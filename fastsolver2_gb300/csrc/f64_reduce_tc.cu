@@ -23,7 +23,7 @@
 // digits.  X's values stay in registers from their load to their digits, and a
 // half's registers are loaded for the next group as soon as they are cut (a
 // first version that loaded the values twice, with eight warps, took 40.3 ms, this
-// order 37.0 at first and now 30.5: the reductions of one factor + solve at N = 2^20,
+// order 37.0 at first and now 31: the reductions of one factor + solve at N = 2^20,
 // leaf 128, rank 32, 64 right-hand sides.  The FP64 FMA kernel took 229.)
 #include <algorithm>
 

@@ -23,6 +23,15 @@
 // against quadruple precision, 32 terms of N(0,1): 1.1e-16, FMA chain 2.0e-16;
 // uniform [0,1): 6.8e-17 against 1.6e-16.
 //
+// Bound.  What holds is relative to the groups, not to each product: with alpha the
+// largest |A(i, .)| of a row and beta the largest |B(., j)| of a column, both balanced
+// (below), and K inner values, |C - A B|(i, j) <= 1.5 K 2^-53 alpha beta + 2^-53 |C|(i, j).
+// An operand at 2^-k of its group's bound keeps 55 - k bits.  An FP64 FMA chain is bound
+// by K 2^-53 sum |a| |b| instead: the same where the values of a row, a column or a group
+// of rows are within a few powers of two once balanced, as bases and right-hand sides
+// are, and smaller where a row's large values meet zeros or small ones.  The products
+// of the factorisations are split so that no tile mixes rows of two kinds (f64_gj.cu).
+//
 // Balance.  Inner index k of A is divided by the power of two of the largest
 // |A(., k)| of the tile and the same index of B multiplied by it (exponents
 // only), so that a factor on inner index k of A with its inverse on B --

@@ -18,7 +18,7 @@
 // of C and A), 6000 at 192, 8200 at 64 and 12300 at 32, where cutting the A
 // tile is not hidden; the issue slots of the epilogue (some 60 instructions a
 // value) are what is left.  At N = 2^20, leaf 128, rank 32, 64 right-hand
-// sides the updates of one factor + solve take 18.5 ms; the FP64 FMA kernel
+// sides the updates of one factor + solve take 18.6 ms; the FP64 FMA kernel
 // (update_nn_kernel) took 196.
 #include <algorithm>
 

@@ -562,7 +562,7 @@ static int cap_apply(hodlr_ctx *h, int l, int C, long long tb_stride, bool trans
 
 // The mixed path at leaf 128, and the FP64 path where it has digit images,
 // factor their leaves by blocked Gauss-Jordan kernels that form the explicit
-// inverses only.  FP64: 8192 leaves of 128 rows take 14 ms so, and 69 in the
+// inverses only.  FP64: 8192 leaves of 128 rows take 15 ms so, and 69 in the
 // register-resident sweep that gives LU and inverse together.
 static bool leaf_inverse_only(const hodlr_ctx *h) {
   return h->mixed ? h->m == 128 && h->Dinv32 : h->Dimg && !h->keep_lu;

@@ -193,7 +193,7 @@ cudaError_t launch_f64_leaf_tc(const unsigned char *img, const int *rows, const 
                                const double *X, long long ldx, double *Y, long long ldy, int ncols, const int *skip,
                                DevStatus *st, cudaStream_t s);
 
-// Dinv = D^-1 of leaves of 64, 128 or 256 rows by blocked Gauss-Jordan, the
+// Dinv = D^-1 of leaves of 64, 128 or 256 rows by blocked elimination, the
 // products on the tensor cores (f64_gj.cu); with LU (m up to 128) the factors and
 // pivots too.  A: workspace [nleaf][m][m], ipiv: [nleaf][m]; scratch: f64_leaf_gj_scratch bytes,
 // 8-byte aligned.
