@@ -21,6 +21,9 @@ static std::mutex g_mu;
 static std::condition_variable g_freed;
 static unsigned long long g_taken = 0;  // bit i: word i, on whichever device
 
+static thread_local long long g_waiting_launches = 0;
+void note_waiting_launch() { ++g_waiting_launches; }
+
 CallStatus::CallStatus() {
   std::unique_lock<std::mutex> lock(g_mu);
   g_freed.wait(lock, [] { return ~g_taken != 0; });
@@ -44,6 +47,7 @@ CallStatus::~CallStatus() {
 
 cudaError_t CallStatus::find() {
   void *p = nullptr;
+  launches_ = g_waiting_launches;
   const cudaError_t e = cudaGetSymbolAddress(&p, g_words);
   if (e == cudaSuccess) word_ = static_cast<DevStatus *>(p) + slot_;
   return e;
@@ -51,7 +55,8 @@ cudaError_t CallStatus::find() {
 
 int CallStatus::finish(const char *call) {
   DevStatus s{};
-  cudaError_t e = cudaMemcpyAsync(&s, word_, sizeof s, cudaMemcpyDeviceToHost, 0);
+  cudaError_t e = cudaSuccess;
+  if (launches_ != g_waiting_launches) e = cudaMemcpyAsync(&s, word_, sizeof s, cudaMemcpyDeviceToHost, 0);
   if (e == cudaSuccess) e = cudaStreamSynchronize(0);
   if (e != cudaSuccess) return set_last_error(HODLR_ERR_CUDA, cudaGetErrorString(e));
   if (s.code == HODLR_OK) {

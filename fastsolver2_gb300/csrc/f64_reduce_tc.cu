@@ -440,6 +440,7 @@ bool f64_reduce_tc_try(const double *V, long long ldv, const double *X, long lon
   a.out = dst;
   a.skip = skip;
   a.st = st;
+  note_waiting_launch();
   err = allow_dyn_smem(f64_reduce_tc_kernel, kSmem);
   if (err != cudaSuccess) return true;
   HODLR_LAUNCH(f64_reduce_tc_kernel, (unsigned)std::min<long long>(a.units, kNumSMs), kThreads, kSmem, s, a);

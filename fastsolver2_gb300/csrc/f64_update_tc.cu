@@ -419,6 +419,7 @@ static cudaError_t launch_kc(const UpdateArgs &a, DevStatus *st, cudaStream_t s)
   if (e != cudaSuccess) return e;
   const int nrt = ceil_div(a.M, 128), nct = ceil_div(a.N, kDigN);
   const int ntiles = nrt * nct * a.nbatch;
+  note_waiting_launch();
   HODLR_LAUNCH(k, (unsigned)std::min(ntiles, kNumSMs), kThreads, Cfg<KC>::kSmem, s, a, nrt, nct, ntiles, st);
   return cudaGetLastError();
 }

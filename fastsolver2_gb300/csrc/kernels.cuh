@@ -22,12 +22,16 @@ class CallStatus {
   CallStatus &operator=(const CallStatus &) = delete;
   cudaError_t find();  // before word()
   DevStatus *word() const { return word_; }
-  int finish(const char *call);  // waits for the stream; the call's status, with the error's text set
+  // Waits for the stream; the call's status, with the error's text set.  The word is
+  // read only if a kernel with waits was launched (note_waiting_launch) in between.
+  int finish(const char *call);
 
  private:
   DevStatus *word_ = nullptr;
   int slot_;
+  long long launches_ = 0;
 };
+void note_waiting_launch();  // this thread launched a kernel that may report HODLR_ERR_TIMEOUT
 
 // Launch-shape choices of the tunable kernels, chosen per handle (per forest
 // of a batch) by the autotuner.  Launches made by a host thread use the
